@@ -244,6 +244,17 @@ __device__ __forceinline__ float2 unpack_bf16x2(uint32_t u) {
     return __bfloat1622float2(v);
 }
 
+// Two fp32 values as three bf16 pairs: x = hi + mid + lo to fp32 precision (3 x 8 bits of mantissa)
+__device__ __forceinline__ void split3(float x0, float x1, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+    hi = pack_bf16x2(x0, x1);
+    float2 h = unpack_bf16x2(hi);
+    x0 -= h.x;
+    x1 -= h.y;
+    mid = pack_bf16x2(x0, x1);
+    h = unpack_bf16x2(mid);
+    lo = pack_bf16x2(x0 - h.x, x1 - h.y);
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

@@ -1,0 +1,277 @@
+// Attention of ONE new query token per sequence over its key / value cache (generation): grouped query heads, head
+// dim 64 or 128, optional sliding window and padding mask.
+//
+// Bound by reading K and V once.  A CTA of four warps owns a slice of the keys of one (batch, K / V head) and serves
+// up to eight query heads of its group from the registers the keys pass through; the slices of one (batch, head)
+// form a cluster and merge their softmax partials through distributed shared memory, so there is one launch and no
+// workspace.  A warp takes 16 keys per step:
+//   scores  mma.sync m16n8k16 with the queries as the 16-row operand (rows 8..15 zero): a lane's 16-byte pieces of a
+//           key ARE its B fragment when the contraction index is numbered accordingly (queries use the same order),
+//           so keys go from global memory to the tensor core without shared memory, shuffles or conversions;
+//   values  the weights stay fp32-exact: p = hi + mid + lo in bf16 (3 x 8 bits of mantissa), hi in rows 0..7, mid in
+//           rows 8..15 of one operand, lo in a second product, all accumulated in fp32; the score fragment's layout is
+//           the weight operand's, and two keys' 16-byte pieces give the value fragments with one byte permute per
+//           register.
+// tcgen05 has nothing to add: one row per head is used, and the bound is HBM.
+// Measured (24 sequences x 3001 keys, 8 K / V heads of 128, 295 MB): 83 us = 3.5 TB/s; the PyTorch statement that served
+// this case before expands K and V to one fp32 copy per query head and took 2640 us.  24 x 501 keys: 41 us (kernel),
+// 1 x 1024 keys: 9.4 us.
+// Included by lme_cuda.cu after m2rnn.cu (mma helper).
+
+namespace lme {
+namespace da {
+
+using m2::mma16816;
+
+constexpr int WARPS = 4;
+constexpr int MAX_SPLITS = 16;
+
+struct Args {
+    const __nv_bfloat16 *q, *k, *v;
+    __nv_bfloat16* out;                     // [B, Hkv * G, D] contiguous
+    const unsigned char* mask;              // [B, Sk] bytes, 0 = hidden, or null
+    long long q_b, q_h, k_b, k_s, k_h, v_b, v_s, v_h, mask_b;   // element strides
+    int first, Sk;                          // keys [first, Sk) are attended
+    int Hkv, G, head_blocks;                // head_blocks = ceil(G / 8): groups of eight query heads
+    float scale;
+};
+
+__device__ __forceinline__ uint4 ld_stream(const __nv_bfloat16* p) {
+    uint4 r;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
+    return r;
+}
+__device__ __forceinline__ uint32_t word(const uint4& u, int i) { return i == 0 ? u.x : i == 1 ? u.y : i == 2 ? u.z : u.w; }
+__device__ __forceinline__ float ld_cluster(const float* p, uint32_t cta) {
+    uint32_t a;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(cta));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+template <int D>
+__global__ void __launch_bounds__(WARPS * 32, 3) decode_attention_kernel(const Args p) {
+    constexpr int KC = D / 32;    // 16-byte pieces of a key per lane
+    constexpr int VC = D / 64;    // 16-byte pieces of a value row per lane
+    __shared__ float s_acc[WARPS][8][D];
+    __shared__ float s_m[WARPS][8], s_l[WARPS][8];
+    __shared__ float c_acc[8][D];
+    __shared__ float c_m[8], c_l[8];
+    const int splits = gridDim.x, split = blockIdx.x;
+    const int kvh = blockIdx.y / p.head_blocks, hb = blockIdx.y % p.head_blocks;
+    const long long b = blockIdx.z;
+    const int heads = min(8, p.G - hb * 8);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+
+    // query fragments; rows >= heads are zero
+    uint32_t qa[D / 16][2];
+    {
+        const __nv_bfloat16* qp = p.q + b * p.q_b + (static_cast<long long>(kvh) * p.G + hb * 8 + g) * p.q_h + 8 * t;
+#pragma unroll
+        for (int j = 0; j < KC; ++j) {
+            uint4 w = make_uint4(0, 0, 0, 0);
+            if (g < heads) w = *reinterpret_cast<const uint4*>(qp + 32 * j);
+            qa[2 * j][0] = w.x;
+            qa[2 * j][1] = w.y;
+            qa[2 * j + 1][0] = w.z;
+            qa[2 * j + 1][1] = w.w;
+        }
+    }
+    const __nv_bfloat16* kb = p.k + b * p.k_b + static_cast<long long>(kvh) * p.k_h + 8 * t;
+    const __nv_bfloat16* vb = p.v + b * p.v_b + static_cast<long long>(kvh) * p.v_h + 8 * g;
+    const unsigned char* mb = p.mask != nullptr ? p.mask + b * p.mask_b : nullptr;
+
+    const int n = p.Sk - p.first;
+    const int per = ((n + splits - 1) / splits + 15) & ~15;
+    const int k0 = p.first + min(n, split * per), k1 = p.first + min(n, (split + 1) * per);
+
+    float acc[D / 8][4];
+#pragma unroll
+    for (int i = 0; i < D / 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    float m = -INFINITY, l = 0.f;     // row g; l is this lane's share
+
+    for (int base = k0 + warp * 16; base < k1; base += WARPS * 16) {
+        uint4 kw[2][KC], vw[4][VC];
+#pragma unroll
+        for (int tile = 0; tile < 2; ++tile) {
+            const int key = min(base + tile * 8 + g, k1 - 1);
+#pragma unroll
+            for (int j = 0; j < KC; ++j) kw[tile][j] = ld_stream(kb + key * p.k_s + 32 * j);
+        }
+        bool ok[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int key = base + (e >> 1) * 8 + 2 * t + (e & 1);
+            ok[e] = key < k1;
+            if (ok[e] && mb != nullptr) ok[e] = mb[key] != 0;
+#pragma unroll
+            for (int j = 0; j < VC; ++j)
+                vw[e][j] = ok[e] ? ld_stream(vb + key * p.v_s + 64 * j) : make_uint4(0, 0, 0, 0);
+        }
+        float s[2][4];
+#pragma unroll
+        for (int tile = 0; tile < 2; ++tile) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) s[tile][i] = 0.f;
+#pragma unroll
+            for (int ks = 0; ks < D / 16; ++ks) {
+                const uint32_t a[4] = {qa[ks][0], 0u, qa[ks][1], 0u};
+                mma16816(s[tile], a, word(kw[tile][ks >> 1], 2 * (ks & 1)), word(kw[tile][ks >> 1], 2 * (ks & 1) + 1));
+            }
+        }
+        float x[4], mx = m;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            x[e] = ok[e] ? s[e >> 1][e & 1] * p.scale : -INFINITY;
+            mx = fmaxf(mx, x[e]);
+        }
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+        if (__any_sync(0xffffffffu, mx > m)) {
+            const float c = m == -INFINITY ? 0.f : __expf(m - mx);
+            l *= c;
+#pragma unroll
+            for (int i = 0; i < D / 8; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] *= c;
+            m = mx;
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            x[e] = x[e] == -INFINITY ? 0.f : __expf(x[e] - m);
+            l += x[e];
+        }
+        uint32_t hi[2], mid[2], lo[2];
+        split3(x[0], x[1], hi[0], mid[0], lo[0]);
+        split3(x[2], x[3], hi[1], mid[1], lo[1]);
+        const uint32_t a0[4] = {hi[0], mid[0], hi[1], mid[1]}, a1[4] = {lo[0], 0u, lo[1], 0u};
+#pragma unroll
+        for (int j = 0; j < VC; ++j)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const uint32_t sel = (i & 1) ? 0x7632u : 0x5410u;
+                const uint32_t b0 = __byte_perm(word(vw[0][j], i >> 1), word(vw[1][j], i >> 1), sel);
+                const uint32_t b1 = __byte_perm(word(vw[2][j], i >> 1), word(vw[3][j], i >> 1), sel);
+                mma16816(acc[j * 8 + i], a0, b0, b1);
+                mma16816(acc[j * 8 + i], a1, b0, b1);
+            }
+    }
+    l += __shfl_xor_sync(0xffffffffu, l, 1);
+    l += __shfl_xor_sync(0xffffffffu, l, 2);
+    // accumulator i of piece j: columns 2t, 2t + 1 of the product are dims 64 j + 8 (2t) + i and 64 j + 8 (2t + 1) + i
+#pragma unroll
+    for (int j = 0; j < VC; ++j)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float* a = acc[j * 8 + i];
+            s_acc[warp][g][64 * j + 16 * t + i] = a[0] + a[2];
+            s_acc[warp][g][64 * j + 16 * t + 8 + i] = a[1] + a[3];
+        }
+    if (t == 0) {
+        s_m[warp][g] = m;
+        s_l[warp][g] = l;
+    }
+    __syncthreads();
+    for (int u = threadIdx.x; u < heads * D; u += WARPS * 32) {
+        const int r = u / D, d = u % D;
+        float M = -INFINITY;
+#pragma unroll
+        for (int w = 0; w < WARPS; ++w) M = fmaxf(M, s_m[w][r]);
+        float a = 0.f, ls = 0.f;
+#pragma unroll
+        for (int w = 0; w < WARPS; ++w) {
+            const float f = s_m[w][r] == -INFINITY ? 0.f : __expf(s_m[w][r] - M);
+            a += f * s_acc[w][r][d];
+            ls += f * s_l[w][r];
+        }
+        c_acc[r][d] = a;
+        if (d == 0) {
+            c_m[r] = M;
+            c_l[r] = ls;
+        }
+    }
+    cluster_sync();
+    for (int u = split * (WARPS * 32) + threadIdx.x; u < heads * D; u += splits * (WARPS * 32)) {
+        const int r = u / D, d = u % D;
+        float M = -INFINITY;
+        for (int c = 0; c < splits; ++c) M = fmaxf(M, ld_cluster(&c_m[r], c));
+        float a = 0.f, ls = 0.f;
+        for (int c = 0; c < splits; ++c) {
+            const float mc = ld_cluster(&c_m[r], c);
+            const float f = mc == -INFINITY ? 0.f : __expf(mc - M);
+            a += f * ld_cluster(&c_acc[r][d], c);
+            ls += f * ld_cluster(&c_l[r], c);
+        }
+        // a row that attends to nothing, or whose scores are not finite, is zero (as in the PyTorch statement)
+        const float o = ls > 0.f && ls < INFINITY ? a / ls : 0.f;
+        p.out[(b * p.Hkv * p.G + static_cast<long long>(kvh) * p.G + hb * 8 + r) * D + d] = __float2bfloat16_rn(o);
+    }
+    cluster_sync();   // the others may still read this CTA's partials
+}
+
+template <int D>
+static int launch_decode_attention(const Args& a, int B, int splits, cudaStream_t st) {
+    auto kern = decode_attention_kernel<D>;
+    static int configured = 0;   // clusters of 16 need an opt-in
+    if (!configured) {
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+            return LME_ERR_LAUNCH;
+        configured = 1;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(splits, a.Hkv * a.head_blocks, B);
+    cfg.blockDim = dim3(WARPS * 32);
+    cfg.stream = st;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = splits;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, a) == cudaSuccess ? LME_OK : LME_ERR_LAUNCH;
+}
+
+}  // namespace da
+}  // namespace lme
+
+extern "C" int lme_decode_attention(const void* q, long long q_b, long long q_h, const void* k, long long k_b,
+                                    long long k_s, long long k_h, const void* v, long long v_b, long long v_s,
+                                    long long v_h, const void* mask, long long mask_b, void* out, int B, int Sk,
+                                    int Hkv, int G, int D, int window, float scale, void* stream) {
+    if (B <= 0 || Hkv <= 0 || G <= 0) return LME_OK;
+    if (Sk <= 0 || window <= 0 || (D != 64 && D != 128)) return LME_ERR_SHAPE;
+    if ((q_b | q_h | k_b | k_s | k_h | v_b | v_s | v_h) % 8) return LME_ERR_SHAPE;
+    if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v)) & 15)
+        return LME_ERR_ALIGN;
+    lme::da::Args a = {};
+    a.q = static_cast<const __nv_bfloat16*>(q);
+    a.k = static_cast<const __nv_bfloat16*>(k);
+    a.v = static_cast<const __nv_bfloat16*>(v);
+    a.out = static_cast<__nv_bfloat16*>(out);
+    a.mask = static_cast<const unsigned char*>(mask);
+    a.q_b = q_b; a.q_h = q_h;
+    a.k_b = k_b; a.k_s = k_s; a.k_h = k_h;
+    a.v_b = v_b; a.v_s = v_s; a.v_h = v_h;
+    a.mask_b = mask_b;
+    a.first = Sk > window ? Sk - window : 0;
+    a.Sk = Sk;
+    a.Hkv = Hkv;
+    a.G = G;
+    a.head_blocks = (G + 7) / 8;
+    a.scale = scale;
+    if (B > 65535 || static_cast<long long>(Hkv) * a.head_blocks > 65535) return LME_ERR_SHAPE;
+    // The keys are split until the grid fills the chip about twice (three CTAs fit an SM), but no slice is shorter
+    // than the 64 keys that the four warps take in one step.
+    const long long rows = static_cast<long long>(B) * Hkv * a.head_blocks;
+    int splits = 1;
+    while (splits < lme::da::MAX_SPLITS && rows * splits < 2 * 3 * 148 && (Sk - a.first) > splits * 64) splits *= 2;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    return D == 64 ? lme::da::launch_decode_attention<64>(a, B, splits, st)
+                   : lme::da::launch_decode_attention<128>(a, B, splits, st);
+}

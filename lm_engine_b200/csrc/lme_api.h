@@ -247,6 +247,14 @@ int lme_pack_rows(const void* x, const int* cu_seqlens, void* out, int B, int S,
 int lme_unpack_rows(const void* packed, const int* cu_seqlens, void* x, int B, int S, long long row_bytes,
                     void* stream);
 
+// Attention of one new token per sequence over its cache (kernels/decode_attention.cu): q [B, Hkv * G, D], k / v
+// [B, Sk, Hkv, D] bf16 with the given element strides, D 64 or 128; mask [B, Sk] bytes (0 = hidden) or null; the last
+// `window` keys are attended.  out [B, Hkv * G, D].
+int lme_decode_attention(const void* q, long long q_b, long long q_h, const void* k, long long k_b, long long k_s,
+                         long long k_h, const void* v, long long v_b, long long v_s, long long v_h, const void* mask,
+                         long long mask_b, void* out, int B, int Sk, int Hkv, int G, int D, int window, float scale,
+                         void* stream);
+
 // Flash-attention forward (kernels/attention.cu): head dim 128, bf16, S_q and S_kv multiples of 128, Hq % Hkv == 0.
 // q [B,S_q,Hq,128], k / v [B,S_kv,Hkv,128] with token pitch ld* elements (heads contiguous inside a token, batches
 // back to back); o [B,S_q,Hq,128] with token pitch ldo; lse fp32 [B,Hq,S_q] or null.  causal aligns the last query

@@ -100,6 +100,7 @@ def cuda_lib() -> ctypes.CDLL:
             "lme_rnn": [P, I, P],
             "lme_attention_fwd": [P, L, P, L, P, L, P, L, P, I, I, I, I, I, I, I, F, P, L, P, I, I, P],
             "lme_attention_bwd": [P, L, P, L, P, L, P, L, P, L, P, P, P, L, P, L, P, L, I, I, I, I, I, I, I, F, P, L, P],
+            "lme_decode_attention": [P, L, L, P, L, L, L, P, L, L, L, P, L, P, I, I, I, I, I, I, F, P],
             "lme_embedding_fwd": [P, P, P, L, I, L, L, P],
             "lme_embedding_bwd": [P, P, P, P, L, I, L, L, P],
             "lme_pack_rows": [P, P, P, I, I, L, L, P],

@@ -44,6 +44,51 @@ def supports(q, k, v, *, causal, sliding_window, attention_mask, cu_seqlens, dro
     return enabled() and (not causal or q.size(1) == k.size(1))
 
 
+def decode_supported(q, k, v, *, causal, sliding_window, attention_mask, cu_seqlens, dropout_p) -> bool:
+    """One new token per sequence over a longer cache, outside autograd (generation): the case that would otherwise
+    run as the PyTorch statement, which expands K and V to fp32 copies per query head.  One key, or a plain
+    non-causal call, keeps the library path that it has."""
+    if not (type(q) is type(k) is type(v) is torch.Tensor and q.is_cuda and q.dim() == 4 and q.size(1) == 1
+            and q.dtype == k.dtype == v.dtype == torch.bfloat16 and q.size(-1) in (64, 128)
+            and k.dim() == 4 and k.shape == v.shape and q.size(-1) == k.size(-1) and q.size(0) == k.size(0)
+            and k.size(2) > 0 and q.size(2) % k.size(2) == 0 and dropout_p == 0 and cu_seqlens is None):
+        return False
+    if torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad):
+        return False
+    if attention_mask is not None and not (type(attention_mask) is torch.Tensor and attention_mask.is_cuda
+                                           and attention_mask.shape == (k.size(0), k.size(1))):
+        return False
+    if torch.autograd.forward_ad._current_level >= 0 or torch._C._functorch.peek_interpreter_stack() is not None:
+        return False        # transforms see the statement
+    plain = sliding_window is None and attention_mask is None
+    return (k.size(1) > 1 and not (plain and not causal) and (sliding_window is None or sliding_window > 0)
+            and q.size(0) <= 65535 and k.size(2) * ((q.size(2) // k.size(2) + 7) // 8) <= 65535)
+
+
+def decode_attention(q, k, v, *, softmax_scale: float, sliding_window: int | None = None, attention_mask=None):
+    """``[B, 1, Hq, D]`` over ``[B, Sk, Hkv, D]`` (csrc/kernels/decode_attention.cu).  The query is the last
+    position, so causality hides nothing; ``sliding_window`` keeps the last that many keys.  Rows that attend to
+    nothing are zero; values of hidden keys are not read into the sum."""
+    def rows(t):
+        ok = t.stride(3) == 1 and t.data_ptr() % 16 == 0 and not any(t.stride(d) % 8 for d in range(3))
+        return t if ok else t.contiguous()
+
+    q, k, v = rows(q), rows(k), rows(v)
+    B, _, Hq, D = q.shape
+    Sk, Hkv = k.size(1), k.size(2)
+    out = torch.empty((B, 1, Hq, D), dtype=q.dtype, device=q.device)
+    mask = None
+    if attention_mask is not None:
+        mask = attention_mask.bool().contiguous()
+    window = Sk if sliding_window is None else min(sliding_window, Sk)
+    _lib.check(_lib.cuda_lib().lme_decode_attention(
+        q.data_ptr(), q.stride(0), q.stride(2), k.data_ptr(), k.stride(0), k.stride(1), k.stride(2), v.data_ptr(),
+        v.stride(0), v.stride(1), v.stride(2), _lib.ptr(mask), Sk, out.data_ptr(), B, Sk, Hkv, Hq // Hkv, D, window,
+        softmax_scale, _lib.stream_ptr()), f"lme_decode_attention B={B} Sk={Sk} Hq={Hq} Hkv={Hkv} D={D}")
+    _lib.count_launch()
+    return out
+
+
 def why_unsupported(q, k, v, *, causal, sliding_window, attention_mask, cu_seqlens, dropout_p) -> str:
     """Short reason why :func:`supports` said no (for the one-time fallback warning)."""
     packed = cu_seqlens is not None
