@@ -84,16 +84,17 @@ __device__ __forceinline__ void tile_coords(int tile, const GemmArgs& p, int& mb
     nb = in / gsz;
 }
 
-// Fused epilogue for 32 consecutive accumulator columns of one output row (held by one thread).
-__device__ __forceinline__ void epilogue_store(const uint32_t (&r)[32], int row, int col0, const GemmArgs& p,
+// Fused epilogue for NC (16 or 32) consecutive accumulator columns of one output row (held by one thread).
+template <int NC>
+__device__ __forceinline__ void epilogue_store(const uint32_t (&r)[NC], int row, int col0, const GemmArgs& p,
                                                bool out_f32, bool accumulate, bool swiglu, long long c_off = 0) {
-        float v[32];
+        float v[NC];
 #pragma unroll
-        for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-        const int ncols = min(32, p.N - col0);  // N % 8 == 0 is enforced on the host
+        for (int i = 0; i < NC; ++i) v[i] = __uint_as_float(r[i]);
+        const int ncols = min(NC, p.N - col0);  // N % 8 == 0 is enforced on the host
         if (p.bias != nullptr) {
 #pragma unroll
-            for (int i = 0; i < 32; i += 8) {
+            for (int i = 0; i < NC; i += 8) {
                 if (i < ncols) {
                     uint4 b = *reinterpret_cast<const uint4*>(p.bias + col0 + i);
                     float2 f;
@@ -108,7 +109,7 @@ __device__ __forceinline__ void epilogue_store(const uint32_t (&r)[32], int row,
             if (p.preact != nullptr) {
                 __nv_bfloat16* pp = p.preact + static_cast<long long>(row) * p.ldp + col0;
 #pragma unroll
-                for (int i = 0; i < 32; i += 8) {
+                for (int i = 0; i < NC; i += 8) {
                     if (i < ncols) {
                         uint4 o;
                         o.x = pack_bf16x2(v[i], v[i + 1]); o.y = pack_bf16x2(v[i + 2], v[i + 3]);
@@ -117,11 +118,11 @@ __device__ __forceinline__ void epilogue_store(const uint32_t (&r)[32], int row,
                     }
                 }
             }
-            // interleaved (gate, up) pairs -> 16 outputs per 32 accumulator columns
+            // interleaved (gate, up) pairs -> one output per two accumulator columns
             __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.C) +
                                  static_cast<long long>(row) * p.ldc + (col0 >> 1);
 #pragma unroll
-            for (int i = 0; i < 32; i += 16) {
+            for (int i = 0; i < NC; i += 16) {
                 if (i < ncols) {
                     float o8[8];
 #pragma unroll
@@ -143,7 +144,7 @@ __device__ __forceinline__ void epilogue_store(const uint32_t (&r)[32], int row,
         if (p.residual != nullptr) {
             const __nv_bfloat16* rp = p.residual + static_cast<long long>(row) * p.ldr + col0;
 #pragma unroll
-            for (int i = 0; i < 32; i += 8) {
+            for (int i = 0; i < NC; i += 8) {
                 if (i < ncols) {
                     uint4 b = *reinterpret_cast<const uint4*>(rp + i);
                     float2 f;
@@ -157,7 +158,7 @@ __device__ __forceinline__ void epilogue_store(const uint32_t (&r)[32], int row,
         if (out_f32) {
             float* out = reinterpret_cast<float*>(p.C) + c_off + static_cast<long long>(row) * p.ldc + col0;
 #pragma unroll
-            for (int i = 0; i < 32; i += 4) {
+            for (int i = 0; i < NC; i += 4) {
                 if (i < ncols) {
                     float4 o = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
                     if (accumulate) {
@@ -171,7 +172,7 @@ __device__ __forceinline__ void epilogue_store(const uint32_t (&r)[32], int row,
             __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.C) + c_off +
                                  static_cast<long long>(row) * p.ldc + col0;
 #pragma unroll
-            for (int i = 0; i < 32; i += 8) {
+            for (int i = 0; i < NC; i += 8) {
                 if (i < ncols) {
                     if (accumulate) {
                         uint4 b = *reinterpret_cast<const uint4*>(out + i);
@@ -549,6 +550,201 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
 }
 
+// ---------------------------------------------------------------------------------------------- split contraction
+// The same product for problems whose 128 x 256 tiles cannot fill the chip (few tokens: generation steps, short
+// prompts, small fine-tuning batches).  128 x 128 tiles, two CTAs per SM, and a cluster of `splits` CTAs per tile,
+// each with a contiguous share of K: the operands of a tile stream through `splits` SMs at once, which is what bounds
+// these shapes (a single CTA waits for its ring: 0.33 us per 64-deep block of K against 0.13 us of multiplication).  Every CTA leaves its fp32 partial tile in its own shared memory
+// (the drained TMA ring), and after a cluster barrier each CTA adds the partials of its share of the rows over
+// distributed shared memory, in rank order, and runs the fused epilogue: one launch, no workspace, deterministic.
+// Times of both kernels and the choice between them: gemm_splits() below.
+static constexpr int SK_BN = 128;
+static constexpr int SK_MAX_SPLITS = 4;
+template <int STAGES>
+struct SplitLayout {
+    static constexpr int A_BYTES = BM * BK * 2;
+    static constexpr int B_BYTES = SK_BN * BK * 2;
+    static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
+    static constexpr int TILES_BYTES = STAGES * STAGE_BYTES;
+    static constexpr int BAR_BYTES = (2 * STAGES + 1) * 8 + 16;
+    static constexpr int TOTAL = TILES_BYTES + BAR_BYTES + 1024;
+    static constexpr int RED_LD = SK_BN + 4;   // floats per row of the partial tile: rows of a warp on distinct banks
+    static_assert(BM * RED_LD * 4 <= TILES_BYTES, "the partial tile reuses the drained ring");
+    static_assert((STAGES == 3 ? 2 : 1) * (TOTAL + 1024) <= 228 * 1024, "CTAs per SM");
+};
+
+__device__ __forceinline__ float4 ld_cluster_f4(const float* p, uint32_t cta) {
+    uint32_t a;
+    float4 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(cta));
+    asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <int STAGES, bool A_MN, bool B_MN>
+__global__ void __launch_bounds__(192, STAGES == 3 ? 2 : 1)
+gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmArgs p,
+                  const int splits) {
+    using L = SplitLayout<STAGES>;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + L::TILES_BYTES);
+    uint64_t* empty_bar = full_bar + STAGES;
+    uint64_t* tfull_bar = empty_bar + STAGES;
+    uint32_t* tmem_base_smem = reinterpret_cast<uint32_t*>(tfull_bar + 1);
+    float* red = reinterpret_cast<float*>(smem);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = blockIdx.x % splits;     // = %cluster_ctarank: the cluster is one-dimensional
+    int mb, nb;
+    tile_coords(blockIdx.x / splits, p, mb, nb);
+    const int m0 = mb * BM, n0 = nb * SK_BN;
+    const int num_kb = (p.K + BK - 1) / BK;
+    const int kb0 = static_cast<int>(static_cast<long long>(num_kb) * rank / splits);
+    const int kb1 = static_cast<int>(static_cast<long long>(num_kb) * (rank + 1) / splits);
+
+    if (threadIdx.x == 0) {
+        tma_prefetch_desc(&tmA);
+        tma_prefetch_desc(&tmB);
+        for (int s = 0; s < STAGES; ++s) {
+            mbar_init(&full_bar[s], 1);
+            mbar_init(&empty_bar[s], 1);
+        }
+        mbar_init(tfull_bar, 1);
+        fence_barrier_init();
+    }
+    if (warp == 1) {
+        tmem_alloc(tmem_base_smem, SK_BN);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_base_smem;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            for (int kb = kb0; kb < kb1; ++kb) {
+                const int it = kb - kb0, s = it % STAGES;
+                if (!mbar_wait(&empty_bar[s], ((it / STAGES) & 1) ^ 1, 500 + s)) break;
+                uint8_t* sa = smem + s * L::STAGE_BYTES;
+                uint8_t* sb = sa + L::A_BYTES;
+                mbar_expect_tx(&full_bar[s], L::STAGE_BYTES);
+                if (A_MN) {
+#pragma unroll
+                    for (int c = 0; c < BM / 64; ++c)
+                        tma_load_2d(sa + c * (BK * 128), &tmA, &full_bar[s], m0 + c * 64, kb * BK);
+                } else {
+                    tma_load_2d(sa, &tmA, &full_bar[s], kb * BK, m0);
+                }
+                if (B_MN) {
+#pragma unroll
+                    for (int c = 0; c < SK_BN / 64; ++c)
+                        tma_load_2d(sb + c * (BK * 128), &tmB, &full_bar[s], n0 + c * 64, kb * BK);
+                } else {
+                    tma_load_2d(sb, &tmB, &full_bar[s], kb * BK, n0);
+                }
+            }
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        if (lane == 0) {
+            const uint32_t idesc = make_idesc(1, 1, A_MN, B_MN, BM, SK_BN);
+            bool ok = true;
+            for (int kb = kb0; kb < kb1; ++kb) {
+                const int it = kb - kb0, s = it % STAGES;
+                if (!mbar_wait(&full_bar[s], (it / STAGES) & 1, 510 + s)) { ok = false; break; }
+                tc_fence_after();
+                const uint32_t sa = smem_u32(smem + s * L::STAGE_BYTES);
+                const uint32_t sb = sa + L::A_BYTES;
+#pragma unroll
+                for (int kk = 0; kk < BK / UMMA_K; ++kk) {
+                    const uint64_t da = A_MN ? make_smem_desc_sw128(sa + kk * (UMMA_K * 128), BK * 128, 1024)
+                                             : make_smem_desc_sw128(sa + kk * (UMMA_K * 2), 16, 1024);
+                    const uint64_t db = B_MN ? make_smem_desc_sw128(sb + kk * (UMMA_K * 128), BK * 128, 1024)
+                                             : make_smem_desc_sw128(sb + kk * (UMMA_K * 2), 16, 1024);
+                    umma_bf16(tmem_base, da, db, idesc, (it > 0 || kk > 0) ? 1u : 0u);
+                }
+                umma_commit(&empty_bar[s]);
+            }
+            if (ok) umma_commit(tfull_bar);
+        }
+        __syncwarp();
+    } else {
+        const int q = warp & 3;
+        const int row = q * 32 + lane;
+        if (mbar_wait(tfull_bar, 0, 520)) {
+            tc_fence_after();
+#pragma unroll 1
+            for (int c = 0; c < SK_BN / 32; ++c) {
+                uint32_t r[32];
+                tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + c * 32, r);
+                tmem_ld_wait();
+                const int col0 = n0 + c * 32;
+                if (m0 + row < p.M && col0 < p.N) {
+                    if (splits == 1) {
+                        epilogue_store(r, m0 + row, col0, p, p.flags & LME_GEMM_OUT_F32, p.flags & LME_GEMM_ACCUMULATE,
+                                       p.flags & LME_GEMM_SWIGLU);
+                    } else {
+                        float* dst = red + row * L::RED_LD + c * 32;
+#pragma unroll
+                        for (int i = 0; i < 32; i += 4)
+                            *reinterpret_cast<uint4*>(dst + i) = make_uint4(r[i], r[i + 1], r[i + 2], r[i + 3]);
+                    }
+                }
+                __syncwarp();
+            }
+        }
+        __syncwarp();
+    }
+    tc_fence_before();
+    if (splits > 1) {
+        cluster_barrier();     // every partial tile is complete and visible
+        // this CTA's share: groups of 16 columns of a row.  The sums go back into the own partial tile (the peers read
+        // other places of it), four columns per thread so that a warp reads whole rows of a peer.
+        const int groups = min(BM, p.M - m0) * (SK_BN / 16);
+        const int g0 = groups * rank / splits, g1 = groups * (rank + 1) / splits;
+        for (int u = 4 * g0 + threadIdx.x; u < 4 * g1; u += blockDim.x) {
+            float* mine = red + u / (SK_BN / 4) * L::RED_LD + u % (SK_BN / 4) * 4;
+            float4 v[SK_MAX_SPLITS];
+#pragma unroll
+            for (int s = 0; s < SK_MAX_SPLITS; ++s)
+                if (s < splits) v[s] = ld_cluster_f4(mine, s);
+#pragma unroll
+            for (int s = 1; s < SK_MAX_SPLITS; ++s)
+                if (s < splits) {
+                    v[0].x += v[s].x; v[0].y += v[s].y; v[0].z += v[s].z; v[0].w += v[s].w;
+                }
+            *reinterpret_cast<float4*>(mine) = v[0];
+        }
+        __syncthreads();
+        for (int u = g0 + threadIdx.x; u < g1; u += blockDim.x) {
+            const int row = u / (SK_BN / 16), c = u % (SK_BN / 16) * 16;
+            if (n0 + c >= p.N) continue;
+            uint32_t r[16];
+#pragma unroll
+            for (int i = 0; i < 16; i += 4) {
+                const uint4 f = *reinterpret_cast<const uint4*>(red + row * L::RED_LD + c + i);
+                r[i] = f.x; r[i + 1] = f.y; r[i + 2] = f.z; r[i + 3] = f.w;
+            }
+            epilogue_store(r, m0 + row, n0 + c, p, p.flags & LME_GEMM_OUT_F32, p.flags & LME_GEMM_ACCUMULATE,
+                           p.flags & LME_GEMM_SWIGLU);
+        }
+        __syncwarp();
+        cluster_barrier();     // the peers have read this CTA's partials
+    }
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc(tmem_base, SK_BN);
+    }
+}
+
 // ----------------------------------------------------------------------------------------------- host side
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -685,6 +881,64 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, GemmArgs& p
     return cudaGetLastError() == cudaSuccess ? LME_OK : LME_ERR_LAUNCH;
 }
 
+template <int STAGES, bool A_MN, bool B_MN>
+static int launch_gemm_split_stages(const CUtensorMap& ta, const CUtensorMap& tb, GemmArgs& p, int splits,
+                             cudaStream_t stream) {
+    auto kern = gemm_split_kernel<STAGES, A_MN, B_MN>;
+    static bool configured = false;
+    if (!configured) {
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitLayout<STAGES>::TOTAL) != cudaSuccess)
+            return LME_ERR_LAUNCH;
+        configured = true;
+    }
+    p.tiles_m = (p.M + BM - 1) / BM;
+    p.tiles_n = (p.N + SK_BN - 1) / SK_BN;
+    p.group_m = 8;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(p.tiles_m) * p.tiles_n * splits);
+    cfg.blockDim = dim3(192);
+    cfg.dynamicSmemBytes = SplitLayout<STAGES>::TOTAL;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = splits;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, ta, tb, static_cast<const GemmArgs>(p), splits) == cudaSuccess
+               ? LME_OK : LME_ERR_LAUNCH;
+}
+
+template <bool A_MN, bool B_MN>
+static int launch_gemm_split(const CUtensorMap& ta, const CUtensorMap& tb, GemmArgs& p, int splits,
+                             cudaStream_t stream) {
+    // up to one CTA per SM: the whole shared memory for one ring, twice as deep
+    const long long ctas = static_cast<long long>((p.M + BM - 1) / BM) * ((p.N + SK_BN - 1) / SK_BN) * splits;
+    return ctas <= num_sms() ? launch_gemm_split_stages<6, A_MN, B_MN>(ta, tb, p, splits, stream)
+                             : launch_gemm_split_stages<3, A_MN, B_MN>(ta, tb, p, splits, stream);
+}
+
+// CTAs per tile for an M x N x K product, 0: the persistent kernel.  A CTA of the split kernel takes 0.33 us per 64-deep
+// block alone on its SM and 0.41 us as one of two, the persistent kernel 0.40 us per block of its wider tile, and adding
+// partial tiles costs 2 to 6 us, so what counts is how many SMs a tile's K streams through.  Measured (B200, operands
+// from HBM, us; persistent / 1 / 2 / 4 CTAs per tile):
+//   M=24   N=4096  K=14336   32 tiles   89.2 / 73.6 / 40.3 / 25.2      M=333 N=2048 K=5632   48 tiles   38.0 / 32.4 / 22.4 / 19.0
+//   M=24   N=6144  K=4096    48 tiles   30.0 / 24.8 / 16.2 / 15.0      M=512 N=2048 K=8192   64 tiles   52.4 / 45.4 / 29.5 / 24.1
+//   M=333  N=3072  K=2048    72 tiles   19.2 / 16.1 / 13.8 / 18.1      M=777 N=2048 K=8192  112 tiles   52.2 / 46.5 / 36.4 / 42.4
+//   M=512  N=4096  K=4096   128 tiles   29.6 / 25.9 / 23.6 / 32.0      M=777 N=2048 K=2048  112 tiles   17.8 / 15.9 / 16.7 / 23.1
+//   M=64   N=28672 K=4096   224 tiles   45.6 / 45.6 / 51.6             M=777 N=4096 K=4096  224 tiles   29.9 / 32.0 / 41.6
+// Four as long as all CTAs are resident at two per SM with room to spare, two while they are and K is long enough to
+// pay for the sum (or one per SM), one while every tile has an SM; from there on the wider tiles of the persistent
+// kernel.  Clusters of eight only won where a whole GPC was free for each and lost elsewhere.
+static int gemm_splits(int M, int N, int K) {
+    const long long tiles = static_cast<long long>((M + BM - 1) / BM) * ((N + SK_BN - 1) / SK_BN);
+    const int blocks = (K + BK - 1) / BK, sms = num_sms();
+    if (tiles > sms) return 0;
+    if (4 * tiles <= 2 * sms - 40 && blocks >= (4 * tiles <= sms ? 12 : 16)) return 4;
+    if (blocks >= (2 * tiles <= sms ? 24 : 48)) return 2;
+    return 1;
+}
+
 }  // namespace lme
 
 using namespace lme;
@@ -698,7 +952,10 @@ extern "C" int lme_gemm_bf16(const void* A, int a_mn_major, long long lda, const
     if ((flags & LME_GEMM_SWIGLU) && (N % 16)) return LME_ERR_SHAPE;
     if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C)) & 15)
         return LME_ERR_ALIGN;
-    const int BN = (N <= 128) ? 128 : 256;
+    // a caller that limits the CTAs (communication kernels run beside this one) keeps the persistent kernel
+    const int splits = max_ctas <= 0 && !(flags & (LME_GEMM_PROBE_NO_LOAD | LME_GEMM_PROBE_NO_MMA))
+                           ? gemm_splits(M, N, K) : 0;
+    const int BN = (N <= 128 || splits > 0) ? 128 : 256;
     CUtensorMap ta, tb;
     int rc;
     // K-major operand [rows, K]: inner = K, box 64 x rows_per_tile.  MN-major operand [K, rows]: inner = rows,
@@ -718,6 +975,12 @@ extern "C" int lme_gemm_bf16(const void* A, int a_mn_major, long long lda, const
     p.scale_a = p.scale_b = nullptr;
     if (max_ctas <= 0) max_ctas = num_sms();
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+if (splits > 0) {
+        if (a_mn_major && b_mn_major) return launch_gemm_split<true, true>(ta, tb, p, splits, st);
+        if (a_mn_major) return launch_gemm_split<true, false>(ta, tb, p, splits, st);
+        if (b_mn_major) return launch_gemm_split<false, true>(ta, tb, p, splits, st);
+        return launch_gemm_split<false, false>(ta, tb, p, splits, st);
+    }
 #define LME_DISPATCH(BN_, ST_)                                                          \
     do {                                                                                \
         if (a_mn_major && b_mn_major) return launch_gemm<BN_, ST_, true, true>(ta, tb, p, max_ctas, st);   \
