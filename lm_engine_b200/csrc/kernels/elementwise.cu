@@ -605,7 +605,9 @@ extern "C" int lme_adamw(float* p, float* m, float* v, const void* g, int g_is_b
     float bc1 = 1.f - powf(b1, static_cast<float>(step));
     float bc2 = 1.f - powf(b2, static_cast<float>(step));
     float bc2_sqrt = sqrtf(bc2);
-    int grid = grid_for((n + 7) / 8, 256, 148 * 8);
+    // One group of eight elements per thread.  Bound by HBM (28 bytes per element); 1184 CTAs that looped over the shard
+    // wrote each stream in 1184 places at once.  109 M elements: 555 -> 513 us, 5.95 TB/s.
+    int grid = grid_for((n + 7) / 8, 256, 0x7fffffff);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (g_is_bf16)
         adamw_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(p, m, v, static_cast<const __nv_bfloat16*>(g),
