@@ -13,9 +13,9 @@
 //           the weight operand's, and two keys' 16-byte pieces give the value fragments with one byte permute per
 //           register.
 // tcgen05 has nothing to add: one row per head is used, and the bound is HBM.
-// Measured (24 sequences x 3001 keys, 8 K / V heads of 128, 295 MB): 83 us = 3.5 TB/s; the PyTorch statement that served
-// this case before expands K and V to one fp32 copy per query head and took 2640 us.  24 x 501 keys: 41 us (kernel),
-// 1 x 1024 keys: 9.4 us.
+// Measured (24 sequences x 3001 keys, 8 K / V heads of 128, 295 MB): 76 us = 3.9 TB/s (84 us without the loads one block
+// ahead); the PyTorch statement that served this case before expands K and V to one fp32 copy per query head and took
+// 2640 us.  What is left is latency: 12 warps per SM at 168 registers, a third of the issue slots used.
 // Included by lme_cuda.cu after m2rnn.cu (mma helper).
 
 namespace lme {
@@ -96,24 +96,37 @@ __global__ void __launch_bounds__(WARPS * 32, 3) decode_attention_kernel(const A
         for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
     float m = -INFINITY, l = 0.f;     // row g; l is this lane's share
 
-    for (int base = k0 + warp * 16; base < k1; base += WARPS * 16) {
-        uint4 kw[2][KC], vw[4][VC];
+    // Loads run one block of 16 keys ahead in the registers that the current block frees: the next keys are requested
+    // right after the scores, the next values (with their mask) right after the products with the weights.
+    uint4 kw[2][KC], vw[4][VC];
+    unsigned ok = 0;            // bit e: the lane's e-th key of the block is attended
+    auto load_keys = [&](int base) {
 #pragma unroll
         for (int tile = 0; tile < 2; ++tile) {
             const int key = min(base + tile * 8 + g, k1 - 1);
 #pragma unroll
             for (int j = 0; j < KC; ++j) kw[tile][j] = ld_stream(kb + key * p.k_s + 32 * j);
         }
-        bool ok[4];
+    };
+    auto load_values = [&](int base) {
+        ok = 0;
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const int key = base + (e >> 1) * 8 + 2 * t + (e & 1);
-            ok[e] = key < k1;
-            if (ok[e] && mb != nullptr) ok[e] = mb[key] != 0;
+            bool in = key < k1;
+            if (in && mb != nullptr) in = mb[key] != 0;
+            ok |= in ? 1u << e : 0u;
 #pragma unroll
             for (int j = 0; j < VC; ++j)
-                vw[e][j] = ok[e] ? ld_stream(vb + key * p.v_s + 64 * j) : make_uint4(0, 0, 0, 0);
+                vw[e][j] = in ? ld_stream(vb + key * p.v_s + 64 * j) : make_uint4(0, 0, 0, 0);
         }
+    };
+    constexpr int STEP = WARPS * 16;
+    if (k0 + warp * 16 < k1) {
+        load_keys(k0 + warp * 16);
+        load_values(k0 + warp * 16);
+    }
+    for (int base = k0 + warp * 16; base < k1; base += STEP) {
         float s[2][4];
 #pragma unroll
         for (int tile = 0; tile < 2; ++tile) {
@@ -125,10 +138,11 @@ __global__ void __launch_bounds__(WARPS * 32, 3) decode_attention_kernel(const A
                 mma16816(s[tile], a, word(kw[tile][ks >> 1], 2 * (ks & 1)), word(kw[tile][ks >> 1], 2 * (ks & 1) + 1));
             }
         }
+        if (base + STEP < k1) load_keys(base + STEP);
         float x[4], mx = m;
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            x[e] = ok[e] ? s[e >> 1][e & 1] * p.scale : -INFINITY;
+            x[e] = (ok >> e & 1) ? s[e >> 1][e & 1] * p.scale : -INFINITY;
             mx = fmaxf(mx, x[e]);
         }
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
@@ -161,6 +175,7 @@ __global__ void __launch_bounds__(WARPS * 32, 3) decode_attention_kernel(const A
                 mma16816(acc[j * 8 + i], a0, b0, b1);
                 mma16816(acc[j * 8 + i], a1, b0, b1);
             }
+        if (base + STEP < k1) load_values(base + STEP);
     }
     l += __shfl_xor_sync(0xffffffffu, l, 1);
     l += __shfl_xor_sync(0xffffffffu, l, 2);
@@ -266,11 +281,11 @@ extern "C" int lme_decode_attention(const void* q, long long q_b, long long q_h,
     a.head_blocks = (G + 7) / 8;
     a.scale = scale;
     if (B > 65535 || static_cast<long long>(Hkv) * a.head_blocks > 65535) return LME_ERR_SHAPE;
-    // The keys are split until the grid fills the chip about twice (three CTAs fit an SM), but no slice is shorter
-    // than the 64 keys that the four warps take in one step.
+    // The keys are split until there is a CTA for every slot of the chip (three fit an SM), but no slice is shorter than
+    // the 64 keys that the four warps take in one step: a slice costs a prologue and a merge of about 4 us.
     const long long rows = static_cast<long long>(B) * Hkv * a.head_blocks;
     int splits = 1;
-    while (splits < lme::da::MAX_SPLITS && rows * splits < 2 * 3 * 148 && (Sk - a.first) > splits * 64) splits *= 2;
+    while (splits < lme::da::MAX_SPLITS && rows * splits < 3 * 148 && (Sk - a.first) > splits * 64) splits *= 2;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     return D == 64 ? lme::da::launch_decode_attention<64>(a, B, splits, st)
                    : lme::da::launch_decode_attention<128>(a, B, splits, st);
