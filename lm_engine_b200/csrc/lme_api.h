@@ -134,6 +134,18 @@ int lme_moe_route_chunks(int total);
 int lme_moe_route_layout(const long long* selected, int total, int E, int* scratch, long long* freq, int* k0, int* kb,
                          int* tile_group, int ntiles, int* slot, void* stream);
 
+// Block-local part of the gated delta rule (kernels/delta_prep.cu): operands of the chain from q, k, v (bf16, strides =
+// nine element strides, (batch, token, head) of each), g and beta (fp32 [B, S, N]); x = the inverse of the 64 x 64
+// unit-triangular factor, kept for the backward, which returns the gradients of all five.
+int lme_delta_prep_fwd(const void* q, const void* k, const void* v, const long long* strides, const float* g,
+                       const float* beta, void* wk, void* qe, void* ke, void* ket, void* qk, float* wv, float* x, float* a,
+                       int B, int S, int N, int K, int V, int l2norm, float scale, void* stream);
+int lme_delta_prep_bwd(const void* q, const void* k, const void* v, const long long* strides, const float* g,
+                       const float* beta, const float* x, const void* du, const void* h, const void* dh,
+                       const float* duh, const float* dqe, const float* dqk, const float* dke, void* dq, void* dk,
+                       void* dv, float* dg, float* dbeta, int B, int S, int N, int K, int V, int l2norm, float scale,
+                       void* stream);
+
 // Inter-chunk chain of the gated delta rule (kernels/delta_rule.cu has the recurrences).  BN = batch * heads, nc chunks
 // of 64 rows, K in {128, 256}, V % 64 == 0.  Forward operands (bf16): wk = W_k [BN][nc][64][K], qe [BN][nc][64][K],
 // ket = K_e^T [BN][nc][K][64], qk [BN][nc][64][64]; fp32: wv [BN][nc][64][V], a [BN][nc], h0 [BN][K][V] or null.

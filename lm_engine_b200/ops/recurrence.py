@@ -8,6 +8,7 @@ flows back through the state at every step - the semantics of lm_engine/modeling
 
 from __future__ import annotations
 
+import ctypes
 import os
 
 import torch
@@ -243,6 +244,119 @@ def delta_chain(Wk, Wv, qe, qk, ke, a, h):
     return delta_chain_reference(Wk, Wv, qe, qk, ke, a, h)
 
 
+class _GatedDeltaBlocks(torch.autograd.Function):
+    """:func:`gated_delta_rule_chunked` on bf16 q, k, v as two kernels each way (csrc/kernels/delta_prep.cu,
+    delta_rule.cu): everything local to a 64-step block in one, the chain over the blocks in the other; the reverse
+    pass has four batched tensor-core GEMMs between them (the products of the chain's U, dU with its states)."""
+
+    @staticmethod
+    def forward(ctx, q, k, v, g, beta, h0, scale, use_qk_l2norm):
+        from . import _lib
+
+        B, S, N, K = q.shape
+        V, L = v.size(-1), CHUNK
+        nc = (S + L - 1) // L
+        bf, f32, dev = torch.bfloat16, torch.float32, q.device
+        n = B * N * nc
+        wk, qe, ke = (torch.empty((n, L, K), dtype=bf, device=dev) for _ in range(3))
+        ket = torch.empty((n, K, L), dtype=bf, device=dev)
+        qk = torch.empty((n, L, L), dtype=bf, device=dev)
+        wv = torch.empty((n, L, V), dtype=f32, device=dev)
+        x = torch.empty((n, L, L), dtype=f32, device=dev)
+        a = torch.empty(n, dtype=f32, device=dev)
+        lib = _lib.cuda_lib()
+        strides = _delta_strides(q, k, v)
+        _lib.check(lib.lme_delta_prep_fwd(
+            q.data_ptr(), k.data_ptr(), v.data_ptr(), strides, g.data_ptr(), beta.data_ptr(), wk.data_ptr(),
+            qe.data_ptr(), ke.data_ptr(), ket.data_ptr(), qk.data_ptr(), wv.data_ptr(), x.data_ptr(), a.data_ptr(), B,
+            S, N, K, V, int(use_qk_l2norm), scale, _lib.stream_ptr()), f"lme_delta_prep_fwd B={B} S={S} N={N} V={V}")
+        y = torch.empty((B, N, nc, L, V), dtype=f32, device=dev)
+        u_all = torch.empty((n, L, V), dtype=bf, device=dev)
+        h_all = torch.empty((n, K, V), dtype=bf, device=dev)
+        h_final = torch.empty((B, N, K, V), dtype=f32, device=dev)
+        h32 = None if h0 is None else h0.float().contiguous()
+        _lib.check(lib.lme_delta_chain_fwd(
+            wk.data_ptr(), qe.data_ptr(), ket.data_ptr(), qk.data_ptr(), wv.data_ptr(), a.data_ptr(), _lib.ptr(h32),
+            y.data_ptr(), u_all.data_ptr(), h_all.data_ptr(), h_final.data_ptr(), B * N, nc, K, V,
+            _lib.stream_ptr()), f"lme_delta_chain_fwd BN={B * N} nc={nc} K={K} V={V}")
+        _lib.count_launch(2)
+        ctx.save_for_backward(q, k, v, g, beta, wk, qe, ke, qk, a, x, u_all, h_all)
+        ctx.cfg = (scale, use_qk_l2norm, h0 is not None)
+        out = torch.empty((B, nc * L, N, V), dtype=bf, device=dev)
+        out.view(B, nc, L, N, V).copy_(y.permute(0, 2, 3, 1, 4))
+        return out[:, :S], h_final
+
+    @staticmethod
+    def backward(ctx, dy, dh_final):
+        from . import _lib
+        from .gemm import _bmm_kernel
+
+        q, k, v, g, beta, wk, qe, ke, qk, a, x, u_all, h_all = ctx.saved_tensors
+        scale, use_qk_l2norm, has_h0 = ctx.cfg
+        B, S, N, K = q.shape
+        V, L = v.size(-1), CHUNK
+        nc = (S + L - 1) // L
+        n = B * N * nc
+        bf, f32, dev = torch.bfloat16, torch.float32, q.device
+        dyb = torch.empty((B, N, nc, L, V), dtype=bf, device=dev)
+        if S < nc * L:
+            dy = torch.nn.functional.pad(dy, (0, 0, 0, 0, 0, nc * L - S))
+        dyb.copy_(dy.reshape(B, nc, L, N, V).permute(0, 3, 1, 2, 4))
+        dyb = dyb.view(n, L, V)
+        dy32 = dyb.float()
+        qkt, qet, wkt = (t.transpose(-1, -2).contiguous() for t in (qk, qe, wk))
+        du, dh = torch.empty_like(u_all), torch.empty_like(h_all)
+        dh0 = torch.empty((B, N, K, V), dtype=f32, device=dev)
+        dhf = None if dh_final is None else dh_final.float().contiguous()
+        lib = _lib.cuda_lib()
+        _lib.check(lib.lme_delta_chain_bwd(
+            qkt.data_ptr(), ke.data_ptr(), qet.data_ptr(), wkt.data_ptr(), dy32.data_ptr(), a.data_ptr(),
+            _lib.ptr(dhf), du.data_ptr(), dh.data_ptr(), dh0.data_ptr(), B * N, nc, K, V, _lib.stream_ptr()),
+            f"lme_delta_chain_bwd BN={B * N} nc={nc} K={K} V={V}")
+        duh = _bmm_kernel(du, h_all, False, False, f32)         # dU h^T = -dW_k
+        dqe = _bmm_kernel(dyb, h_all, False, False, f32)        # dy h^T
+        dqk = _bmm_kernel(dyb, u_all, False, False, f32)        # dy U^T
+        dke = _bmm_kernel(u_all, dh, False, False, f32)         # U dh^T
+        dq, dk = (torch.empty((B, S, N, K), dtype=bf, device=dev) for _ in range(2))
+        dv = torch.empty((B, S, N, V), dtype=bf, device=dev)
+        dg, dbeta = (torch.empty((B, S, N), dtype=f32, device=dev) for _ in range(2))
+        _lib.check(lib.lme_delta_prep_bwd(
+            q.data_ptr(), k.data_ptr(), v.data_ptr(), _delta_strides(q, k, v), g.data_ptr(), beta.data_ptr(),
+            x.data_ptr(), du.data_ptr(), h_all.data_ptr(), dh.data_ptr(), duh.data_ptr(), dqe.data_ptr(),
+            dqk.data_ptr(), dke.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), dg.data_ptr(),
+            dbeta.data_ptr(), B, S, N, K, V, int(use_qk_l2norm), scale, _lib.stream_ptr()),
+            f"lme_delta_prep_bwd B={B} S={S} N={N} V={V}")
+        _lib.count_launch(2)
+        return dq, dk, dv, dg, dbeta, (dh0 if has_h0 else None), None, None
+
+
+def _delta_strides(*tensors):
+    """Batch, token and head strides of ``[B, S, N, X]`` tensors as a C array."""
+    flat = [t.stride(d) for t in tensors for d in range(3)]
+    return (ctypes.c_longlong * len(flat))(*flat)
+
+
+def _delta_operand(t: torch.Tensor) -> torch.Tensor:
+    """Rows that the kernels read in 16-byte pieces (any batch / token / head pitch that keeps them aligned)."""
+    ok = t.stride(3) == 1 and t.data_ptr() % 16 == 0 and not any(t.stride(d) % 8 for d in range(3))
+    return t if ok else t.contiguous()
+
+
+def gated_delta_blocks_usable(q, k, v, g, beta) -> bool:
+    """bf16 q / k / v of one head count on the GPU with the widths of the chain kernels; other inputs keep the
+    tensor-operation form of the block-local part."""
+    B, S, N, K = q.shape
+    return (q.is_cuda and q.dtype == k.dtype == v.dtype == torch.bfloat16 and K in (128, 256)
+            and v.size(-1) % 64 == 0 and v.size(-1) > 0 and q.shape == k.shape and v.shape[:3] == q.shape[:3]
+            and g.shape == beta.shape == q.shape[:3] and 0 < B * N <= 65535 and S > 0)
+
+
+def gated_delta_rule_blocks(q, k, v, g, beta, scale=None, h0=None, use_qk_l2norm: bool = True):
+    scale = q.size(-1) ** -0.5 if scale is None else scale
+    return _GatedDeltaBlocks.apply(_delta_operand(q), _delta_operand(k), _delta_operand(v), g.float().contiguous(),
+                                   beta.float().contiguous(), h0, float(scale), bool(use_qk_l2norm))
+
+
 def linear_attention_scan(q, k, v, h0=None, attention_multiplier: float = 1.0):
     """``y_t = q_t . h_{t-1}`` (state read before the update), ``h_t = h_{t-1} + k_t (x) v_t``; fp32 state."""
     B, S, _, K = q.shape
@@ -334,7 +448,9 @@ def gated_delta_rule(q, k, v, g, beta, scale=None, h0=None, use_qk_l2norm: bool 
     if q.size(1) < 8:
         return gated_delta_rule_scan(q, k, v, g, beta, scale, h0, use_qk_l2norm)
     if q.is_cuda and q.size(-1) in (128, 256) and v.size(-1) % 64 == 0:
-        # the chain over 64-step blocks is one kernel each way
+        # the chain over 64-step blocks is one kernel each way, and so is the block-local part on bf16 inputs
+        if gated_delta_blocks_usable(q, k, v, g, beta):
+            return gated_delta_rule_blocks(q, k, v, g, beta, scale, h0, use_qk_l2norm)
         return gated_delta_rule_chunked(q, k, v, g, beta, scale, h0, use_qk_l2norm, chunk=64)
     # the loop over blocks is the sequential (launch-bound) part and the block-local work is cheap: long sequences
     # take large blocks (the intra-block cost grows with the block length, the number of loop trips falls with it)
