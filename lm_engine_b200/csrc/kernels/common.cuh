@@ -233,6 +233,9 @@ __host__ __device__ constexpr uint32_t make_idesc(uint32_t a_fmt, uint32_t b_fmt
 }
 
 // ------------------------------------------------------------------ small numeric helpers
+// sigmoid with the approximate exponential and reciprocal (a few ulp of fp32; an IEEE division per element costs more
+// instructions than the rest of a bandwidth-bound element-wise kernel)
+__device__ __forceinline__ float sigmoid_fast(float x) { return __fdividef(1.0f, 1.0f + __expf(-x)); }
 __device__ __forceinline__ float silu_f(float x) { return x / (1.0f + __expf(-x)); }
 
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {

@@ -86,8 +86,8 @@ def cuda_lib() -> ctypes.CDLL:
             "lme_decode_attention": [P, L, L, P, L, L, L, P, L, L, L, P, L, P, I, I, I, I, I, I, F, P],
             "lme_delta_chain_fwd": [P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, P],
             "lme_delta_chain_bwd": [P, P, P, P, P, P, P, P, P, P, I, I, I, I, P],
-            "lme_causal_conv1d_fwd": [P, P, P, P, P, I, I, I, I, I, P],
-            "lme_causal_conv1d_bwd": [P, P, P, P, P, P, P, P, P, I, I, I, I, I, P],
+            "lme_causal_conv1d_fwd": [P, L, L, P, P, P, P, I, I, I, I, I, P],
+            "lme_causal_conv1d_bwd": [P, L, L, P, P, P, P, P, P, P, P, I, I, I, I, I, P],
             "lme_reduce_slices": [P, I, P, L, I, F, I, P],
             "lme_reduce_scatter_peers": [P, P, P, I, I, I, P, L, I, F, I, P, I, P],
             "lme_sum_partials": [P, I, P, I, P],

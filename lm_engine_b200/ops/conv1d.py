@@ -32,15 +32,17 @@ class _CausalConv1d(torch.autograd.Function):
     def forward(ctx, x, weight, bias, initial_state, silu: bool):
         from . import _lib
 
-        x = x.contiguous()
         B, S, C = x.shape
         K = weight.size(1)
+        # the four-tap kernels read a slice of wider rows in place (aligned to 16 bytes)
+        if K != 4 or x.stride(2) != 1 or x.stride(1) % 8 or x.stride(0) % 8 or x.data_ptr() % 16:
+            x = x.contiguous()
         w = weight.contiguous()
         init = initial_state.to(x.dtype).contiguous() if initial_state is not None else None
-        y = torch.empty_like(x)
-        _lib.check(_lib.cuda_lib().lme_causal_conv1d_fwd(x.data_ptr(), w.data_ptr(), _lib.ptr(bias), _lib.ptr(init),
-                                                         y.data_ptr(), B, S, C, K, int(silu), _lib.stream_ptr()),
-                   f"lme_causal_conv1d_fwd B={B} S={S} C={C} K={K}")
+        y = torch.empty((B, S, C), dtype=x.dtype, device=x.device)
+        _lib.check(_lib.cuda_lib().lme_causal_conv1d_fwd(x.data_ptr(), x.stride(0), x.stride(1), w.data_ptr(),
+                                                         _lib.ptr(bias), _lib.ptr(init), y.data_ptr(), B, S, C, K,
+                                                         int(silu), _lib.stream_ptr()), f"lme_causal_conv1d_fwd B={B} S={S} C={C} K={K}")
         _lib.count_launch()
         ctx.save_for_backward(x, w, bias, init)
         ctx.silu = silu
@@ -54,13 +56,13 @@ class _CausalConv1d(torch.autograd.Function):
         B, S, C = x.shape
         K = w.size(1)
         dy = dy.contiguous()
-        dx = torch.empty_like(x)
+        dx = torch.empty((B, S, C), dtype=x.dtype, device=x.device)
         dw = torch.zeros((C, K), dtype=torch.float32, device=x.device)
         db = torch.zeros(C, dtype=torch.float32, device=x.device) if bias is not None else None
         dinit = (torch.empty((B, C, K - 1), dtype=torch.float32, device=x.device)
                  if init is not None and ctx.needs_input_grad[3] else None)
         _lib.check(_lib.cuda_lib().lme_causal_conv1d_bwd(
-            x.data_ptr(), w.data_ptr(), _lib.ptr(bias), _lib.ptr(init), dy.data_ptr(), dx.data_ptr(), dw.data_ptr(),
+            x.data_ptr(), x.stride(0), x.stride(1), w.data_ptr(), _lib.ptr(bias), _lib.ptr(init), dy.data_ptr(), dx.data_ptr(), dw.data_ptr(),
             _lib.ptr(db), _lib.ptr(dinit), B, S, C, K, int(ctx.silu), _lib.stream_ptr()),
             f"lme_causal_conv1d_bwd B={B} S={S} C={C} K={K}")
         _lib.count_launch()
