@@ -342,6 +342,10 @@ int lme_swiglu_bwd(const void* x, const void* dy, void* dx, long long T, long lo
 // the same on 128-row tiles of which only those with tile_group[tile] >= 0 are read and written (T % 128 == 0)
 int lme_swiglu_bwd_tiles(const void* x, const void* dy, void* dx, long long T, long long I, const int* tile_group,
                          void* stream);
+// out = y * silu(gate) on [T, I] (gate rows gate_stride elements apart), and its gradients
+int lme_silu_mul_fwd(const void* y, const void* gate, long long gate_stride, void* out, long long T, int I, void* stream);
+int lme_silu_mul_bwd(const void* dout, const void* y, const void* gate, long long gate_stride, void* dy, void* dgate,
+                     long long T, int I, void* stream);
 // fused QKV split + NeoX rotary embedding (inverse = 1: backward, packs dq/dk/dv into dqkv).  cos_t / sin_t are
 // [max_pos, rope_dim]; pos (optional) has T entries, else position = t % S.  A position outside the table sets the
 // status word (STATUS_BOUNDS) instead of reading out of bounds.

@@ -9,11 +9,11 @@ from __future__ import annotations
 
 import torch.nn as nn
 
+from ...ops.activation import silu_mul
 from ...ops.recurrence import gated_delta_rule
 from ...parallel.manager import ProcessGroupManager
 from ...utils import divide_if_divisible
 from ..context import AttentionMaskInfo, GenerationCache, PositionInfo, resolve_attention_and_position_info
-from .activations import silu
 from .conv import DepthwiseCausalConvolution
 from .decay_gate import SoftplusDecayGate
 from .init_utils import std_for_linear
@@ -87,6 +87,6 @@ class GatedDeltaNet(nn.Module):
             cache_params.update(self.layer_idx, "conv", c, GenerationCache.REPLACE, num_tokens_added=S)
             cache_params.update(self.layer_idx, "state", h, GenerationCache.REPLACE)
         if self.use_gate:
-            o = o * silu(gate.view(*o.shape[:-2], -1, self.v_head_dim))
+            o = silu_mul(o.flatten(-2, -1), gate).view(o.shape)
         o = self.o_norm(o)
         return self.o_proj(o.flatten(-2, -1))

@@ -6,12 +6,13 @@ from __future__ import annotations
 
 import torch.nn as nn
 
+from ...ops.activation import silu_mul
 from ...ops.recurrence import linear_attention
 from ...parallel.manager import ProcessGroupManager
 from ...parameter import mark_parameter_as_mup_learning_rate
 from ...utils import divide_if_divisible
 from ..context import AttentionMaskInfo, GenerationCache, PositionInfo, resolve_attention_and_position_info
-from .activations import is_glu, silu
+from .activations import is_glu
 from .conv import DepthwiseCausalConvolution
 from .init_utils import std_for_linear
 from .linear import ParameterizedLinear
@@ -80,5 +81,5 @@ class LinearAttention(nn.Module):
             cache_params.update(self.layer_idx, "conv", c, GenerationCache.REPLACE, num_tokens_added=S)
             cache_params.update(self.layer_idx, "state", h, GenerationCache.REPLACE)
         g = g.repeat_interleave(self.num_heads // self.num_g_heads, dim=-1)
-        y = y.flatten(-2, -1) * silu(g)
+        y = silu_mul(y.flatten(-2, -1), g)
         return self.output_projection(self.g_norm(y))

@@ -7,6 +7,7 @@ from __future__ import annotations
 import torch
 import torch.nn as nn
 
+from ...ops.activation import silu_mul
 from ...ops.recurrence import m2rnn
 from ...parallel.manager import ProcessGroupManager
 from ...parallel.sequence_pipeline import sequence_pipeline
@@ -17,7 +18,7 @@ from ...parameter import (
 )
 from ...utils import divide_if_divisible
 from ..context import AttentionMaskInfo, GenerationCache, PositionInfo, resolve_attention_and_position_info
-from .activations import is_glu, silu
+from .activations import is_glu
 from .conv import DepthwiseCausalConvolution
 from .decay_gate import SoftplusDecayGate
 from .init_utils import std_for_linear
@@ -122,5 +123,5 @@ class M2RNN(nn.Module):
             cache_params.update(self.layer_idx, "conv", c, GenerationCache.REPLACE, num_tokens_added=S)
             cache_params.update(self.layer_idx, "state", h, GenerationCache.REPLACE)
         g = g.repeat_interleave(self.num_heads // self.num_g_heads, dim=-1)
-        y = y.flatten(-2, -1) * silu(g)
+        y = silu_mul(y.flatten(-2, -1), g)
         return self.output_projection(self.g_norm(y))

@@ -8,6 +8,7 @@ from __future__ import annotations
 import torch
 import torch.nn as nn
 
+from ...ops.activation import silu_mul
 from ...ops.ssd import ssd_chunk_scan, ssd_context_parallel_initial_state, ssd_recurrent_step
 from ...parallel.manager import ProcessGroupManager
 from ...parameter import (
@@ -18,7 +19,6 @@ from ...parameter import (
 from ...utils import divide_if_divisible
 from ..config import Mamba2Args
 from ..context import AttentionMaskInfo, GenerationCache, PositionInfo, resolve_attention_and_position_info
-from .activations import silu
 from .conv import DepthwiseCausalConvolution, apply_mask_to_padding_states
 from .decay_gate import SoftplusDecayGate
 from .init_utils import std_for_linear
@@ -114,5 +114,5 @@ class Mamba2(nn.Module):
         y = y.reshape(b, S, I)
         if layout is not None:
             y = layout.pack(y)
-        y = y * silu(gate)
+        y = silu_mul(y, gate)
         return self.out_proj(self.norm(y))

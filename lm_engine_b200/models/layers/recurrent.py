@@ -7,6 +7,7 @@ from __future__ import annotations
 import torch
 import torch.nn as nn
 
+from ...ops.activation import silu_mul
 from ...ops.recurrence import gru, rnn
 from ...parallel.manager import ProcessGroupManager
 from ...parameter import (
@@ -16,7 +17,7 @@ from ...parameter import (
 )
 from ...utils import divide_if_divisible
 from ..context import AttentionMaskInfo, GenerationCache, PositionInfo, resolve_attention_and_position_info
-from .activations import get_activation_function, is_glu, silu
+from .activations import get_activation_function, is_glu
 from .conv import DepthwiseCausalConvolution
 from .init_utils import std_for_linear
 from .linear import ParameterizedLinear
@@ -92,7 +93,7 @@ class _RecurrentBase(nn.Module):
         if cache_params is not None:
             cache_params.update(self.layer_idx, "conv", c, GenerationCache.REPLACE, num_tokens_added=S)
             cache_params.update(self.layer_idx, "state", h, GenerationCache.REPLACE)
-        y = y.flatten(-2, -1) * silu(g)
+        y = silu_mul(y.flatten(-2, -1), g)
         return self.output_projection(self.norm(y))
 
     def extra_repr(self) -> str:

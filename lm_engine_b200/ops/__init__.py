@@ -1,7 +1,7 @@
 """Operators: hand-written sm_100a kernels behind autograd functions, each with a PyTorch reference statement that
 is both the CPU path and the numerical oracle of the tests."""
 
-from .activation import swiglu_backward, swiglu_packed, swiglu_packed_reference
+from .activation import silu_mul, swiglu_backward, swiglu_packed, swiglu_packed_reference
 from .cross_entropy import cross_entropy_sum
 from .gemm import bmm, bmm_reference, gemm, gemm_reference, linear, linear_swiglu
 from .norm import rmsnorm, rmsnorm_reference

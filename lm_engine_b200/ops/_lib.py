@@ -116,6 +116,8 @@ def cuda_lib() -> ctypes.CDLL:
             "lme_rmsnorm_bwd": [P, P, P, P, P, P, P, P, I, I, I, P],
             "lme_swiglu_fwd": [P, P, L, L, P],
             "lme_swiglu_bwd": [P, P, P, L, L, P],
+            "lme_silu_mul_fwd": [P, P, L, P, L, I, P],
+            "lme_silu_mul_bwd": [P, P, P, L, P, P, L, I, P],
             "lme_swiglu_bwd_tiles": [P, P, P, L, L, P, P],
             "lme_qkv_rope": [P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, P],
             "lme_ce_stats": [P, L, P, P, P, P, I, I, I, P],

@@ -73,3 +73,41 @@ def swiglu_backward(preact: torch.Tensor, dy: torch.Tensor, tile_group: torch.Te
     out[..., ::2] = d * u * s * (1 + g * (1 - s))
     out[..., 1::2] = d * g * s
     return out.to(preact.dtype)
+
+
+class _SiLUMul(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, y, gate):
+        I = y.size(-1)
+        y2 = y.reshape(-1, I).contiguous()
+        out = torch.empty_like(y2)
+        _lib.check(_lib.cuda_lib().lme_silu_mul_fwd(y2.data_ptr(), gate.data_ptr(), gate.stride(-2), out.data_ptr(),
+                                                    y2.size(0), I, _lib.stream_ptr()), "lme_silu_mul_fwd")
+        _lib.count_launch()
+        ctx.save_for_backward(y2, gate)
+        ctx.shape = y.shape
+        return out.view(y.shape)
+
+    @staticmethod
+    def backward(ctx, dout):
+        y2, gate = ctx.saved_tensors
+        T, I = y2.shape
+        d2 = dout.reshape(T, I).contiguous()
+        dy, dg = torch.empty_like(y2), torch.empty_like(y2)
+        _lib.check(_lib.cuda_lib().lme_silu_mul_bwd(d2.data_ptr(), y2.data_ptr(), gate.data_ptr(), gate.stride(-2),
+                                                    dy.data_ptr(), dg.data_ptr(), T, I, _lib.stream_ptr()),
+                   "lme_silu_mul_bwd")
+        _lib.count_launch()
+        return dy.view(ctx.shape), dg.view(gate.shape)
+
+
+def silu_mul(y: torch.Tensor, gate: torch.Tensor) -> torch.Tensor:
+    """``y * silu(gate)`` (fp32 inside, one rounding); ``gate`` may be a slice of wider rows."""
+    if (y.is_cuda and gate.is_cuda and y.dtype == gate.dtype == torch.bfloat16 and y.shape == gate.shape
+            and y.dim() >= 2 and y.size(-1) % 8 == 0 and y.numel() > 0):
+        rows = gate.stride(-1) == 1 and gate.stride(-2) % 8 == 0 and gate.data_ptr() % 16 == 0
+        pitch = gate.stride(-2)
+        for d in range(gate.dim() - 2, 0, -1):       # one pitch from row to row through the leading dimensions
+            rows = rows and (gate.size(d - 1) == 1 or gate.stride(d - 1) == gate.size(d) * gate.stride(d))
+        return _SiLUMul.apply(y, gate if rows and pitch > 0 else gate.contiguous())
+    return y * torch.nn.functional.silu(gate.float()).to(gate.dtype)
