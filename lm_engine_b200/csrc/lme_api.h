@@ -293,24 +293,37 @@ int lme_attention_bwd(const void* q, long long ldq, const void* k, long long ldk
                       int Hq, int Hkv, int causal, int window, float scale, const int* cu_seqlens,
                       long long total_tokens, void* stream);
 
-// Element-wise glue of the chunked SSD scan (kernels/ssd.cu), BC = batch x chunks, L % 32 == 0, P in {32, 64, 128}:
-//   prep    (mode 0) xh[BC,N,L,P] = x[BC,L,N,P] dt[BC,L,N];  xwT[BC,N,P,L] = x dt tail, transposed          (bf16)
-//           (mode 1) dx, ddt, dtail from dxh (fp32 [BC,N,L,P]) and dxwT (bf16 [BC,N,P,L])
-//   combine (mode 0) y[BC,L,N,P] = yin[BC,N,L,P] + off[BC,G,L,(N/G)P] ecum[BC,L,N] + D[n] x                 (bf16 out)
-//           (mode 1) dyin, doff (bf16), decum, dDp[BC,L,N] (fp32 row sums of dy x), dx = D dy
-int lme_ssd_prep(const void* x, const float* dt, const float* tail, void* xh, void* xwT, const float* dxh,
-                 const void* dxwT, void* dx, float* ddt, float* dtail, long long BC, int N, int L, int P, int mode,
-                 void* stream);
-int lme_ssd_combine(const float* yin, const float* off, const float* ecum, const float* D, const void* x, void* y,
-                    const void* dy, void* dyin, void* doff, float* decum, float* dDp, void* dx, long long BC, int N,
-                    int L, int G, int P, int mode, void* stream);
+// Decays and element-wise glue of the chunked SSD scan (kernels/ssd.cu), BC = batch x chunks, L % 32 == 0, L <= 1024,
+// P in {32, 64, 128}; x rows (all heads of a token) xs elements apart.
+//   decay    ct = inclusive sums of dt A inside the chunk, dtt = dt, tail = exp(last - ct) ([BC,N,L]), ecum = exp(ct)
+//            ([BC,L,N]), decay [BC,N] = exp(last); the backward turns the gradients into ddt and per-chunk dA, dD
+//   prep     xh[BC,N,L,P] = x[BC,L,N,P] dt;  xwT[BC,N,P,L] = x dt tail, transposed (bf16; dt, tail as [BC,N,L])
+//   combine  y[BC,L,N,P] = yin[BC,N,L,P] + off[BC,G,L,(N/G)P] ecum[BC,L,N] + D[n] x                         (bf16)
+int lme_ssd_decay_fwd(const float* dt, const float* A, float* ct, float* dtt, float* tail, float* ecum, float* decay,
+                      long long BC, int N, int L, void* stream);
+int lme_ssd_decay_bwd(const float* dtt, const float* A, const float* tail, const float* ecum, const float* decay,
+                      const float* sy, const float* decum, const float* ddt0, const float* sw, const float* sh,
+                      const float* ddecay_parts, int parts, const float* dDp, float* ddt, float* dA_part,
+                      float* dD_part, long long BC, int N, int L, void* stream);
+int lme_ssd_prep_fwd(const void* x, long long xs, const float* dt, const float* tail, void* xh, void* xwT, long long BC,
+                     int N, int L, int P, void* stream);
+int lme_ssd_prep_bwd(const void* x, long long xs, const float* dt, const float* tail, const float* dxh,
+                     const void* dxwT, const void* dy, const float* D, void* dx, float* ddt0, float* sw, float* sh,
+                     long long BC, int N, int L, int P, void* stream);
+int lme_ssd_combine_fwd(const float* yin, const float* off, const float* ecum, const float* D, const void* x,
+                        long long xs, void* y, long long BC, int N, int L, int G, int P, void* stream);
+int lme_ssd_combine_bwd(const void* dy, const float* yin, const float* off, const float* ecum, const void* x,
+                        long long xs, void* dyin, void* doff, float* sy, float* decum, float* dDp, long long BC, int N,
+                        int L, int G, int P, void* stream);
 // Chunk-boundary recurrence h_{c+1} = decay[c] h_c + states[c] per (batch, head), E = P * Sd elements (E % 4 == 0):
 // forward writes the state at every chunk start (bf16, and fp32 when h0_f32 != null) and the final state; backward
-// (E <= 16384) returns dstates, ddecay and (optionally) dh_init from dh0 / dh_final (either may be null).
+// returns dstates (fp32 or bf16), ddecay as (E + 127) / 128 partial sums per row and (optionally) dh_init from dh0 /
+// dh_final (either may be null).
 int lme_ssd_boundary_fwd(const float* states, const float* decay, const float* h_init, void* h0_bf16, float* h0_f32,
                          float* h_final, int B, int NC, int N, int E, void* stream);
 int lme_ssd_boundary_bwd(const float* dh0, const float* dh_final, const float* h0_f32, const float* decay,
-                         float* dstates, float* ddecay, float* dh_init, int B, int NC, int N, int E, void* stream);
+                         void* dstates, int dstates_bf16, float* ddecay_parts, float* dh_init, int B, int NC, int N,
+                         int E, void* stream);
 
 
 // max |x| of n bf16 values, max-combined into *amax (which must hold 0 or an earlier running maximum).

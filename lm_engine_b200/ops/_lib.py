@@ -94,10 +94,14 @@ def cuda_lib() -> ctypes.CDLL:
             "lme_set_peer_wait_limit_ms": [L],
             "lme_ssd_decay_matrix": [P, P, P, L, I, I, I, P],
             "lme_ssd_dcb": [P, P, P, L, I, I, I, P],
-            "lme_ssd_prep": [P, P, P, P, P, P, P, P, P, P, L, I, I, I, I, P],
-            "lme_ssd_combine": [P, P, P, P, P, P, P, P, P, P, P, P, L, I, I, I, I, I, P],
+            "lme_ssd_decay_fwd": [P, P, P, P, P, P, P, L, I, I, P],
+            "lme_ssd_decay_bwd": [P, P, P, P, P, P, P, P, P, P, P, I, P, P, P, P, L, I, I, P],
+            "lme_ssd_prep_fwd": [P, L, P, P, P, P, L, I, I, I, P],
+            "lme_ssd_prep_bwd": [P, L, P, P, P, P, P, P, P, P, P, P, L, I, I, I, P],
+            "lme_ssd_combine_fwd": [P, P, P, P, P, L, P, L, I, I, I, I, P],
+            "lme_ssd_combine_bwd": [P, P, P, P, P, L, P, P, P, P, P, L, I, I, I, I, P],
             "lme_ssd_boundary_fwd": [P, P, P, P, P, P, I, I, I, I, P],
-            "lme_ssd_boundary_bwd": [P, P, P, P, P, P, P, I, I, I, I, P],
+            "lme_ssd_boundary_bwd": [P, P, P, P, P, I, P, P, I, I, I, I, P],
             "lme_gemm_bf16_batched": [P, I, L, L, P, I, L, L, P, L, L, I, I, I, I, I, I, P],
             "lme_m2rnn": [P, I, P],
             "lme_rnn": [P, I, P],

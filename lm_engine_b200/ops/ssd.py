@@ -91,86 +91,6 @@ class _IntraChunk(torch.autograd.Function):
         return dCB, dct, dxdt
 
 
-class _ScanPrep(torch.autograd.Function):
-    """``xh[b,c,n,l,:] = x dt`` and ``xwT[b,c,n,:,l] = x dt tail`` (bf16 operands of the intra-chunk and the
-    chunk-state products) from ``x [b, nc, L, N, P]`` bf16 and ``dt``, ``tail [b, nc, L, N]`` fp32, in one kernel;
-    one more for all three gradients."""
-
-    @staticmethod
-    def forward(ctx, x, dt, tail):
-        from . import _lib
-
-        b, nc, L, N, P = x.shape
-        x, dt, tail = x.contiguous(), dt.contiguous(), tail.contiguous()
-        xh = torch.empty((b, nc, N, L, P), dtype=torch.bfloat16, device=x.device)
-        xwT = torch.empty((b, nc, N, P, L), dtype=torch.bfloat16, device=x.device)
-        _lib.check(_lib.cuda_lib().lme_ssd_prep(x.data_ptr(), dt.data_ptr(), tail.data_ptr(), xh.data_ptr(),
-                                                xwT.data_ptr(), None, None, None, None, None, b * nc, N, L, P, 0,
-                                                _lib.stream_ptr()), "lme_ssd_prep")
-        _lib.count_launch()
-        ctx.save_for_backward(x, dt, tail)
-        return xh, xwT
-
-    @staticmethod
-    def backward(ctx, dxh, dxwT):
-        from . import _lib
-
-        x, dt, tail = ctx.saved_tensors
-        b, nc, L, N, P = x.shape
-        dxh = (torch.zeros((b, nc, N, L, P), dtype=torch.float32, device=x.device) if dxh is None
-               else dxh.float().contiguous())
-        dxwT = (torch.zeros((b, nc, N, P, L), dtype=torch.bfloat16, device=x.device) if dxwT is None
-                else dxwT.to(torch.bfloat16).contiguous())
-        dx = torch.empty_like(x)
-        ddt, dtail = torch.empty_like(dt), torch.empty_like(tail)
-        _lib.check(_lib.cuda_lib().lme_ssd_prep(x.data_ptr(), dt.data_ptr(), tail.data_ptr(), None, None,
-                                                dxh.data_ptr(), dxwT.data_ptr(), dx.data_ptr(), ddt.data_ptr(),
-                                                dtail.data_ptr(), b * nc, N, L, P, 1, _lib.stream_ptr()),
-                   "lme_ssd_prep(backward)")
-        _lib.count_launch()
-        return dx, ddt, dtail
-
-
-class _ScanCombine(torch.autograd.Function):
-    """``y = yin^T + off ecum + D x`` in bf16 ``[b, nc, L, N, P]`` from the intra-chunk result ``yin [b,nc,N,L,P]``,
-    the carried-state product ``off [b,nc,G,L,(N/G) P]`` (both fp32), ``ecum [b,nc,L,N]``, ``D [N]`` and ``x``."""
-
-    @staticmethod
-    def forward(ctx, yin, off, ecum, D, x):
-        from . import _lib
-
-        b, nc, L, N, P = x.shape
-        G = off.size(2)
-        yin, off, ecum, D, x = yin.contiguous(), off.contiguous(), ecum.contiguous(), D.contiguous(), x.contiguous()
-        y = torch.empty_like(x)
-        _lib.check(_lib.cuda_lib().lme_ssd_combine(yin.data_ptr(), off.data_ptr(), ecum.data_ptr(), D.data_ptr(),
-                                                   x.data_ptr(), y.data_ptr(), None, None, None, None, None, None,
-                                                   b * nc, N, L, G, P, 0, _lib.stream_ptr()), "lme_ssd_combine")
-        _lib.count_launch()
-        ctx.save_for_backward(off, ecum, D, x)
-        return y
-
-    @staticmethod
-    def backward(ctx, dy):
-        from . import _lib
-
-        off, ecum, D, x = ctx.saved_tensors
-        b, nc, L, N, P = x.shape
-        G = off.size(2)
-        dy = dy.to(torch.bfloat16).contiguous()
-        dyin = torch.empty((b, nc, N, L, P), dtype=torch.bfloat16, device=x.device)
-        doff = torch.empty(off.shape, dtype=torch.bfloat16, device=x.device)
-        decum = torch.empty_like(ecum)
-        dDp = torch.empty_like(ecum)
-        dx = torch.empty_like(x)
-        _lib.check(_lib.cuda_lib().lme_ssd_combine(None, off.data_ptr(), ecum.data_ptr(), D.data_ptr(), x.data_ptr(),
-                                                   None, dy.data_ptr(), dyin.data_ptr(), doff.data_ptr(),
-                                                   decum.data_ptr(), dDp.data_ptr(), dx.data_ptr(), b * nc, N, L, G,
-                                                   P, 1, _lib.stream_ptr()), "lme_ssd_combine(backward)")
-        _lib.count_launch()
-        return dyin, doff, decum, dDp.sum((0, 1, 2)), dx
-
-
 class _BoundaryScan(torch.autograd.Function):
     """``h_{c+1} = decay[c] h_c + S_c`` over the chunks of every (batch, head) in one kernel each way.  Returns the
     state at every chunk start in bf16 (``[b, nc, N, P, Sd]``, the operand of the carried-state product) and the
@@ -204,19 +124,20 @@ class _BoundaryScan(torch.autograd.Function):
         dh0 = None if dh0 is None else dh0.float().contiguous()
         dhf = None if dhf is None else dhf.float().contiguous()
         dstates = torch.empty_like(h0f)
-        ddecay = torch.empty_like(decay)
+        parts = torch.empty((*decay.shape, (P * Sd + 127) // 128), dtype=torch.float32, device=h0f.device)
         dinit = torch.empty((b, N, P, Sd), dtype=torch.float32, device=h0f.device) if ctx.has_init else None
         _lib.check(_lib.cuda_lib().lme_ssd_boundary_bwd(_lib.ptr(dh0), _lib.ptr(dhf), h0f.data_ptr(),
-                                                        decay.data_ptr(), dstates.data_ptr(), ddecay.data_ptr(),
+                                                        decay.data_ptr(), dstates.data_ptr(), 0, parts.data_ptr(),
                                                         _lib.ptr(dinit), b, nc, N, P * Sd, _lib.stream_ptr()),
                    "lme_ssd_boundary_bwd")
         _lib.count_launch()
-        return dstates, ddecay, dinit
+        return dstates, parts.sum(-1), dinit
 
 
-def scan_glue_eligible(x: torch.Tensor, L: int) -> bool:
-    return (x.is_cuda and x.dtype == torch.bfloat16 and L % 32 == 0 and L <= 1024 and x.size(-1) in (32, 64, 128)
-            and FUSED_INTRA_CHUNK)
+def scan_glue_eligible(x: torch.Tensor, L: int, Sd: int) -> bool:
+    b, S, N, P = x.shape
+    return (x.is_cuda and x.dtype == torch.bfloat16 and L % 32 == 0 and L <= 1024 and P in (32, 64, 128)
+            and Sd % 8 == 0 and 0 < b * N <= 65535 and 0 < b * ((S + L - 1) // L) <= 65535 and FUSED_INTRA_CHUNK)
 
 
 def _intra_chunk_fused(Cc, Bc, ct, xdt):
@@ -241,24 +162,22 @@ def ssd_chunk_scan(x, dt, A, B, C, D, chunk_size: int, initial_state=None):
     dtype = x.dtype
     L = chunk_size
     pad = (L - S % L) % L
-    kernels = scan_glue_eligible(x, L)          # then x is consumed in bf16 by the glue kernels: no fp32 copy of it
-    xf, dtf, Bf, Cf = (None if kernels else x.float()), dt.float(), B.float(), C.float()
+    if scan_glue_eligible(x, L, Sd):
+        return _chunk_scan_kernels(x, dt, A, B, C, D, L, initial_state)
+    xf, dtf, Bf, Cf = x.float(), dt.float(), B.float(), C.float()
     if pad:
-        if not kernels:
-            xf = torch.nn.functional.pad(xf, (0, 0, 0, 0, 0, pad))
+        xf = torch.nn.functional.pad(xf, (0, 0, 0, 0, 0, pad))
         dtf = torch.nn.functional.pad(dtf, (0, 0, 0, pad))
         Bf = torch.nn.functional.pad(Bf, (0, 0, 0, 0, 0, pad))
         Cf = torch.nn.functional.pad(Cf, (0, 0, 0, 0, 0, pad))
     nc = (S + pad) // L
-    xc = None if kernels else xf.view(b, nc, L, N, P)
+    xc = xf.view(b, nc, L, N, P)
     dtc = dtf.view(b, nc, L, N)
     Bc = Bf.view(b, nc, L, G, Sd)
     Cc = Cf.view(b, nc, L, G, Sd)
     rep = N // G
     dA = dtc * A.float()                                      # [b, nc, L, N]
     cum = torch.cumsum(dA, dim=2)
-    if kernels:
-        return _chunk_scan_kernels(x, pad, dtc, cum, Bc, Cc, D, initial_state, b, S, nc, L, N, P, G, Sd)
     # ---- intra-chunk: y[t] = sum_{s<=t} exp(cum[t]-cum[s]) (C_t.B_s) dt_s x_s
     ct = cum.permute(0, 1, 3, 2)                              # [b, nc, N, L]
     xdt = xc * dtc[..., None]                                 # [b, nc, L, N, P]
@@ -301,33 +220,140 @@ def ssd_chunk_scan(x, dt, A, B, C, D, chunk_size: int, initial_state=None):
     return y.to(dtype), h
 
 
-def _chunk_scan_kernels(x, pad, dtc, cum, Bc, Cc, D, initial_state, b, S, nc, L, N, P, G, Sd):
-    """The CUDA composition of :func:`ssd_chunk_scan`: the element-wise passes are two kernels (:class:`_ScanPrep`,
-    :class:`_ScanCombine`), the L x L part is :class:`_IntraChunk`, every product is the batched tcgen05 GEMM
-    (:func:`lm_engine_b200.ops.gemm.bmm`), the recurrence over chunk boundaries is :class:`_BoundaryScan`; only
-    per-(token, head) scalars (decays, their cumulative sums) stay PyTorch ops."""
-    rep = N // G
-    xb = torch.nn.functional.pad(x, (0, 0, 0, 0, 0, pad)) if pad else x
-    xc = xb.reshape(b, nc, L, N, P)
-    tail = torch.exp(cum[:, :, -1:, :] - cum)                 # [b, nc, L, N]
-    xh, xwT = _ScanPrep.apply(xc, dtc, tail)
-    # intra-chunk
-    Cg = Cc.permute(0, 1, 3, 2, 4).to(torch.bfloat16).contiguous()        # [b, nc, G, L, Sd]
-    Bg = Bc.permute(0, 1, 3, 2, 4).to(torch.bfloat16).contiguous()
-    from .gemm import bmm
+class _ChunkScan(torch.autograd.Function):
+    """The CUDA composition of :func:`ssd_chunk_scan` for whole chunks.  Per-(token, head) decays, the element-wise
+    passes, the decay matrix and the recurrence over chunk boundaries are the kernels of csrc/kernels/ssd.cu, every
+    product is the batched tcgen05 GEMM on bf16 operands with fp32 results.  One function instead of a chain of them:
+    what the kernels hand to the products' gradients is already in the type that they read, where autograd would cast
+    every gradient to its forward tensor's type and back.  x, B and C may be slices of wider rows."""
 
-    CB = bmm(Cg.view(b * nc * G, L, Sd), Bg.view(b * nc * G, L, Sd),
-             out_dtype=torch.bfloat16).view(b, nc, G, L, L)              # C B^T per (batch, chunk, group)
-    yin = _IntraChunk.apply(CB, cum.permute(0, 1, 3, 2), xh)             # [b, nc, N, L, P] fp32
-    # chunk summaries S_c [b, nc, G, rep*P, Sd] (the heads of a group folded into the GEMM's M dimension);
-    # B_c is [L, Sd] = [K, N]: the MN-major operand
-    states = bmm(xwT.view(b * nc * G, rep * P, L), Bg.view(b * nc * G, L, Sd), b_mn=True).view(b, nc, N, P, Sd)
-    chunk_decay = torch.exp(cum[:, :, -1, :])                 # [b, nc, N]
-    h0, h = _BoundaryScan.apply(states, chunk_decay, initial_state)      # [b, nc, N, P, Sd] bf16, [b, N, P, Sd]
-    # carried-state contribution C_t . h_c: the states [rep*P, Sd] are the K-major B operand as they are
-    off = bmm(Cg.view(b * nc * G, L, Sd), h0.view(b * nc * G, rep * P, Sd)).view(b, nc, G, L, rep * P)
-    y = _ScanCombine.apply(yin, off, torch.exp(cum), D.float(), xc)
-    return y.reshape(b, nc * L, N, P)[:, :S], h
+    @staticmethod
+    def forward(ctx, x, dt, A, B, C, D, L, h_init):
+        from . import _lib
+        from .gemm import _bmm_kernel
+
+        b, S, N, P = x.shape
+        G, Sd = B.shape[-2:]
+        nc, rep, bf, f32, dev = S // L, N // G, torch.bfloat16, torch.float32, x.device
+        bc = b * nc
+        lib, st = _lib.cuda_lib(), _lib.stream_ptr()
+
+        def new(*shape, dtype=f32):
+            return torch.empty(shape, dtype=dtype, device=dev)
+
+        ct, dtt, tail, ecum, decay = new(bc, N, L), new(bc, N, L), new(bc, N, L), new(bc, L, N), new(bc, N)
+        _lib.check(lib.lme_ssd_decay_fwd(dt.data_ptr(), A.data_ptr(), ct.data_ptr(), dtt.data_ptr(), tail.data_ptr(),
+                                         ecum.data_ptr(), decay.data_ptr(), bc, N, L, st), "lme_ssd_decay_fwd")
+        xs = x.stride(1)
+        xh, xwT = new(bc, N, L, P, dtype=bf), new(bc, N, P, L, dtype=bf)
+        _lib.check(lib.lme_ssd_prep_fwd(x.data_ptr(), xs, dtt.data_ptr(), tail.data_ptr(), xh.data_ptr(),
+                                        xwT.data_ptr(), bc, N, L, P, st), "lme_ssd_prep_fwd")
+        Bg, Cg = _chunk_rows(B, bc, L), _chunk_rows(C, bc, L)                # [bc * G, L, Sd]
+        CB = _bmm_kernel(Cg, Bg, False, False, bf)                           # C B^T  [bc * G, L, L]
+        M = new(bc, N, L, L, dtype=bf)
+        _lib.check(lib.lme_ssd_decay_matrix(CB.data_ptr(), ct.data_ptr(), M.data_ptr(), bc, N, G, L, st),
+                   "lme_ssd_decay_matrix")
+        yin = _bmm_kernel(M.view(-1, L, L), xh.view(-1, L, P), False, True, f32)          # [bc * N, L, P]
+        # chunk summaries S_c [rep * P, Sd]: the heads of a group folded into the GEMM's M dimension
+        states = _bmm_kernel(xwT.view(bc * G, rep * P, L), Bg, False, True, f32)
+        h0, hf = new(b, nc, N, P, Sd, dtype=bf), new(b, N, P, Sd)
+        keep = any(ctx.needs_input_grad)      # the backward pass walks the fp32 states
+        h0f = new(b, nc, N, P, Sd) if keep else None
+        h_init = None if h_init is None else h_init.float().contiguous()
+        _lib.check(lib.lme_ssd_boundary_fwd(states.data_ptr(), decay.data_ptr(), _lib.ptr(h_init), h0.data_ptr(),
+                                            _lib.ptr(h0f), hf.data_ptr(), b, nc, N, P * Sd, st),
+                   "lme_ssd_boundary_fwd")
+        h0 = h0.view(bc * G, rep * P, Sd)
+        off = _bmm_kernel(Cg, h0, False, False, f32)                         # C_t . h_c  [bc * G, L, rep * P]
+        y = new(b, S, N, P, dtype=bf)
+        _lib.check(lib.lme_ssd_combine_fwd(yin.data_ptr(), off.data_ptr(), ecum.data_ptr(), D.data_ptr(), x.data_ptr(),
+                                           xs, y.data_ptr(), bc, N, L, G, P, st), "lme_ssd_combine_fwd")
+        _lib.count_launch(5)
+        if keep:
+            ctx.save_for_backward(x, dtt, A, D, Bg, Cg, ct, tail, ecum, decay, xh, xwT, M, yin, off, h0, h0f)
+        ctx.cfg = (L, G, Sd, h_init is not None)
+        return y, hf
+
+    @staticmethod
+    def backward(ctx, dy, dhf):
+        from . import _lib
+        from .gemm import _bmm_kernel
+
+        x, dtt, A, D, Bg, Cg, ct, tail, ecum, decay, xh, xwT, M, yin, off, h0, h0f = ctx.saved_tensors
+        L, G, Sd, has_init = ctx.cfg
+        b, S, N, P = x.shape
+        nc, rep, bf, f32, dev = S // L, N // G, torch.bfloat16, torch.float32, x.device
+        bc = b * nc
+        lib, st = _lib.cuda_lib(), _lib.stream_ptr()
+
+        def new(*shape, dtype=f32):
+            return torch.empty(shape, dtype=dtype, device=dev)
+
+        dy, xs = dy.to(bf).contiguous(), x.stride(1)
+        dyin, doff = new(bc * N, L, P, dtype=bf), new(bc * G, L, rep * P, dtype=bf)
+        sy, decum, dDp, ddt0, sw, sh, ddt = (new(bc * L * N) for _ in range(7))
+        _lib.check(lib.lme_ssd_combine_bwd(dy.data_ptr(), yin.data_ptr(), off.data_ptr(), ecum.data_ptr(), x.data_ptr(),
+                                           xs, dyin.data_ptr(), doff.data_ptr(), sy.data_ptr(), decum.data_ptr(),
+                                           dDp.data_ptr(), bc, N, L, G, P, st), "lme_ssd_combine_bwd")
+        xv = xh.view(-1, L, P)
+        dM = _bmm_kernel(dyin, xv, False, False, bf)                         # dy xdt^T  [bc * N, L, L]
+        dxh = _bmm_kernel(M.view(-1, L, L), dyin, True, True, f32)           # M^T dy
+        dCB = new(bc * G, L, L, dtype=bf)
+        _lib.check(lib.lme_ssd_dcb(dM.data_ptr(), ct.data_ptr(), dCB.data_ptr(), bc, N, G, L, st), "lme_ssd_dcb")
+        # carried state: off = C h0^T
+        dh0 = _bmm_kernel(doff, Cg, True, True, f32)                         # [bc * G, rep * P, Sd]
+        dhf = None if dhf is None else dhf.float().contiguous()
+        dstates = new(bc * G, rep * P, Sd, dtype=bf)
+        parts = (P * Sd + 127) // 128
+        ddecay = new(bc, N, parts)
+        dinit = new(b, N, P, Sd) if has_init else None
+        _lib.check(lib.lme_ssd_boundary_bwd(dh0.data_ptr(), _lib.ptr(dhf), h0f.data_ptr(), decay.data_ptr(),
+                                            dstates.data_ptr(), 1, ddecay.data_ptr(), _lib.ptr(dinit), b, nc, N, P * Sd,
+                                            st), "lme_ssd_boundary_bwd")
+        # chunk summaries: S = xw^T B
+        dxwT = _bmm_kernel(dstates, Bg, False, False, bf)                    # [bc * G, rep * P, L]
+        dB = _bmm_kernel(xwT.view(bc * G, rep * P, L), dstates, True, True, f32) + _bmm_kernel(dCB, Cg, True, True, f32)
+        dC = _bmm_kernel(doff, h0, False, True, f32) + _bmm_kernel(dCB, Bg, False, True, f32)
+        dx = new(b, S, N, P, dtype=bf)
+        _lib.check(lib.lme_ssd_prep_bwd(x.data_ptr(), xs, dtt.data_ptr(), tail.data_ptr(), dxh.data_ptr(),
+                                        dxwT.data_ptr(), dy.data_ptr(), D.data_ptr(), dx.data_ptr(), ddt0.data_ptr(),
+                                        sw.data_ptr(), sh.data_ptr(), bc, N, L, P, st), "lme_ssd_prep_bwd")
+        dA, dD = new(bc, N), new(bc, N)
+        _lib.check(lib.lme_ssd_decay_bwd(dtt.data_ptr(), A.data_ptr(), tail.data_ptr(), ecum.data_ptr(),
+                                         decay.data_ptr(), sy.data_ptr(), decum.data_ptr(), ddt0.data_ptr(),
+                                         sw.data_ptr(), sh.data_ptr(), ddecay.data_ptr(), parts, dDp.data_ptr(), ddt.data_ptr(),
+                                         dA.data_ptr(), dD.data_ptr(), bc, N, L, st), "lme_ssd_decay_bwd")
+        _lib.count_launch(5)
+
+        def tokens(t):        # [bc * G, L, Sd] -> [b, S, G, Sd]
+            return t.view(bc, G, L, Sd).permute(0, 2, 1, 3).reshape(b, S, G, Sd).to(bf)
+
+        return dx, ddt.view(b, S, N), dA.sum(0), tokens(dB), tokens(dC), dD.sum(0), None, dinit
+
+
+def _chunk_rows(t: torch.Tensor, bc: int, L: int) -> torch.Tensor:
+    """B or C ``[b, S, G, Sd]`` as one ``[L, Sd]`` operand per (chunk, group); a single group is read in place."""
+    b, S, G, Sd = t.shape
+    if G == 1 and t.stride(3) == 1 and (b == 1 or t.stride(0) == S * t.stride(1)):
+        return t.as_strided((bc, L, Sd), (L * t.stride(1), t.stride(1), 1), t.storage_offset())
+    return t.reshape(bc, L, G, Sd).permute(0, 2, 1, 3).reshape(bc * G, L, Sd).contiguous()
+
+
+def _chunk_scan_kernels(x, dt, A, B, C, D, L: int, initial_state):
+    """Pads to whole chunks (padded steps have dt = 0: decay 1, no input) and runs :class:`_ChunkScan`."""
+    b, S, N, P = x.shape
+    bf = torch.bfloat16
+    pad = (L - S % L) % L
+    x, B, C, dt = x, B.to(bf), C.to(bf), dt.float()
+    if pad:
+        x, B, C = (torch.nn.functional.pad(t, (0, 0, 0, 0, 0, pad)) for t in (x, B, C))
+        dt = torch.nn.functional.pad(dt, (0, 0, 0, pad))
+    # rows of x: heads contiguous inside a token, one pitch from token to token over the whole batch
+    ok = (x.stride(3) == 1 and x.stride(2) == P and x.stride(1) % 8 == 0 and x.data_ptr() % 16 == 0
+          and (b == 1 or x.stride(0) == x.size(1) * x.stride(1)))
+    y, h = _ChunkScan.apply(x if ok else x.contiguous(), dt.contiguous(), A.float().contiguous(), B, C,
+                            D.float().contiguous(), L, initial_state)
+    return y[:, :S], h
 
 
 def ssd_context_parallel_initial_state(final_zero_init: torch.Tensor, total_decay: torch.Tensor, group) -> torch.Tensor:
