@@ -8,7 +8,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("with_res", [False, True])
-@pytest.mark.parametrize("T,H", [(1, 8), (3, 128), (3600, 256), (4001, 512), (445, 520), (1790, 1024), (2, 1032),
+@pytest.mark.parametrize("T,H", [(1, 8), (3, 128), (3600, 256), (4001, 512), (445, 520), (1790, 1024), (1776, 2048), (1777, 2048), (1800, 8200), (2, 1032),
                                  (900, 2056), (1335, 4096), (333, 6144), (31, 8200), (450, 16384)])
 def test_rmsnorm_layouts(T, H, with_res):
     from lm_engine_b200.ops import _lib, rmsnorm
