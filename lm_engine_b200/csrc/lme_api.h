@@ -159,13 +159,15 @@ int lme_delta_chain_bwd(const void* qkt, const void* ke, const void* qet, const 
                         const float* a, const float* dh_final, void* du_all, void* dh_all, float* dh0, int BN, int nc,
                         int K, int V, void* stream);
 
-// Depthwise causal convolution on channel-last bf16 activations x [B, S, C], weight [C, K] (K <= 8), optional bias [C]
+// Depthwise causal convolution on channel-last bf16 activations x [B, S, C] (rows x_t and batches x_b elements apart,
+// multiples of 8; contiguous unless K = 4), weight [C, K] (K <= 8, 8-byte aligned for K = 4), optional bias [C]
 // and initial state init [B, C, K-1] (the inputs before t = 0); silu != 0 fuses the activation.  Backward recomputes
 // the pre-activation; dw [C, K] / dbias [C] are fp32 accumulators the caller zeroes, dinit [B, C, K-1] is written.
-int lme_causal_conv1d_fwd(const void* x, long long x_b, long long x_t, const void* w, const void* bias, const void* init, void* y, int B, int S,
-                          int C, int K, int silu, void* stream);
-int lme_causal_conv1d_bwd(const void* x, long long x_b, long long x_t, const void* w, const void* bias, const void* init, const void* dy, void* dx,
-                          float* dw, float* dbias, float* dinit, int B, int S, int C, int K, int silu, void* stream);
+int lme_causal_conv1d_fwd(const void* x, long long x_b, long long x_t, const void* w, const void* bias,
+                          const void* init, void* y, int B, int S, int C, int K, int silu, void* stream);
+int lme_causal_conv1d_bwd(const void* x, long long x_b, long long x_t, const void* w, const void* bias,
+                          const void* init, const void* dy, void* dx, float* dw, float* dbias, float* dinit, int B,
+                          int S, int C, int K, int silu, void* stream);
 
 // out (=|+=) scale * sum of nsrc <= 8 local slices of n elements (bf16 or fp32, fp32 accumulation): the reduction
 // half of a reduce-scatter whose peer slices were pulled by copy engines.

@@ -165,6 +165,12 @@ def ptr(t: torch.Tensor | None) -> int | None:
     return None if t is None else t.data_ptr()
 
 
+def aligned(t: torch.Tensor) -> torch.Tensor:
+    """``t`` contiguous and on a 16-byte boundary (kernels with 16-byte accesses; a contiguous view may start anywhere)."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 def raise_peer_wait_limit() -> None:
     """Cross-GPU waits inside kernels (flags that another rank writes) get ``LME_PEER_WAIT_MS`` (default 60 s)
     instead of the 2 s of waits that only this GPU's work feeds: ranks drift apart by seconds around first-step

@@ -79,7 +79,7 @@ class _SiLUMul(torch.autograd.Function):
     @staticmethod
     def forward(ctx, y, gate):
         I = y.size(-1)
-        y2 = y.reshape(-1, I).contiguous()
+        y2 = _lib.aligned(y.reshape(-1, I))
         out = torch.empty_like(y2)
         _lib.check(_lib.cuda_lib().lme_silu_mul_fwd(y2.data_ptr(), gate.data_ptr(), gate.stride(-2), out.data_ptr(),
                                                     y2.size(0), I, _lib.stream_ptr()), "lme_silu_mul_fwd")
@@ -92,7 +92,7 @@ class _SiLUMul(torch.autograd.Function):
     def backward(ctx, dout):
         y2, gate = ctx.saved_tensors
         T, I = y2.shape
-        d2 = dout.reshape(T, I).contiguous()
+        d2 = _lib.aligned(dout.reshape(T, I))
         dy, dg = torch.empty_like(y2), torch.empty_like(y2)
         _lib.check(_lib.cuda_lib().lme_silu_mul_bwd(d2.data_ptr(), y2.data_ptr(), gate.data_ptr(), gate.stride(-2),
                                                     dy.data_ptr(), dg.data_ptr(), T, I, _lib.stream_ptr()),
@@ -109,5 +109,5 @@ def silu_mul(y: torch.Tensor, gate: torch.Tensor) -> torch.Tensor:
         pitch = gate.stride(-2)
         for d in range(gate.dim() - 2, 0, -1):       # one pitch from row to row through the leading dimensions
             rows = rows and (gate.size(d - 1) == 1 or gate.stride(d - 1) == gate.size(d) * gate.stride(d))
-        return _SiLUMul.apply(y, gate if rows and pitch > 0 else gate.contiguous())
+        return _SiLUMul.apply(y, gate if rows and pitch >= gate.size(-1) else _lib.aligned(gate))
     return y * torch.nn.functional.silu(gate.float()).to(gate.dtype)

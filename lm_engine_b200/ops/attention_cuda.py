@@ -71,7 +71,7 @@ def decode_attention(q, k, v, *, softmax_scale: float, sliding_window: int | Non
     nothing are zero; values of hidden keys are not read into the sum."""
     def rows(t):
         ok = t.stride(3) == 1 and t.data_ptr() % 16 == 0 and not any(t.stride(d) % 8 for d in range(3))
-        return t if ok else t.contiguous()
+        return t if ok else _lib.aligned(t)
 
     q, k, v = rows(q), rows(k), rows(v)
     B, _, Hq, D = q.shape

@@ -37,7 +37,7 @@ class _CausalConv1d(torch.autograd.Function):
         # the four-tap kernels read a slice of wider rows in place (aligned to 16 bytes)
         if K != 4 or x.stride(2) != 1 or x.stride(1) % 8 or x.stride(0) % 8 or x.data_ptr() % 16:
             x = x.contiguous()
-        w = weight.contiguous()
+        w = _lib.aligned(weight)
         init = initial_state.to(x.dtype).contiguous() if initial_state is not None else None
         y = torch.empty((B, S, C), dtype=x.dtype, device=x.device)
         _lib.check(_lib.cuda_lib().lme_causal_conv1d_fwd(x.data_ptr(), x.stride(0), x.stride(1), w.data_ptr(),

@@ -338,8 +338,10 @@ def _delta_strides(*tensors):
 
 def _delta_operand(t: torch.Tensor) -> torch.Tensor:
     """Rows that the kernels read in 16-byte pieces (any batch / token / head pitch that keeps them aligned)."""
+    from ._lib import aligned
+
     ok = t.stride(3) == 1 and t.data_ptr() % 16 == 0 and not any(t.stride(d) % 8 for d in range(3))
-    return t if ok else t.contiguous()
+    return t if ok else aligned(t)
 
 
 def gated_delta_blocks_usable(q, k, v, g, beta) -> bool:

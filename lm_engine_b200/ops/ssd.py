@@ -289,7 +289,7 @@ class _ChunkScan(torch.autograd.Function):
         def new(*shape, dtype=f32):
             return torch.empty(shape, dtype=dtype, device=dev)
 
-        dy, xs = dy.to(bf).contiguous(), x.stride(1)
+        dy, xs = _lib.aligned(dy.to(bf)), x.stride(1)
         dyin, doff = new(bc * N, L, P, dtype=bf), new(bc * G, L, rep * P, dtype=bf)
         sy, decum, dDp, ddt0, sw, sh, ddt = (new(bc * L * N) for _ in range(7))
         _lib.check(lib.lme_ssd_combine_bwd(dy.data_ptr(), yin.data_ptr(), off.data_ptr(), ecum.data_ptr(), x.data_ptr(),
@@ -334,9 +334,12 @@ class _ChunkScan(torch.autograd.Function):
 def _chunk_rows(t: torch.Tensor, bc: int, L: int) -> torch.Tensor:
     """B or C ``[b, S, G, Sd]`` as one ``[L, Sd]`` operand per (chunk, group); a single group is read in place."""
     b, S, G, Sd = t.shape
-    if G == 1 and t.stride(3) == 1 and (b == 1 or t.stride(0) == S * t.stride(1)):
+    if (G == 1 and t.stride(3) == 1 and t.stride(1) % 8 == 0 and t.data_ptr() % 16 == 0
+            and (b == 1 or t.stride(0) == S * t.stride(1))):
         return t.as_strided((bc, L, Sd), (L * t.stride(1), t.stride(1), 1), t.storage_offset())
-    return t.reshape(bc, L, G, Sd).permute(0, 2, 1, 3).reshape(bc * G, L, Sd).contiguous()
+    from ._lib import aligned
+
+    return aligned(t.reshape(bc, L, G, Sd).permute(0, 2, 1, 3).reshape(bc * G, L, Sd))
 
 
 def _chunk_scan_kernels(x, dt, A, B, C, D, L: int, initial_state):
@@ -344,14 +347,16 @@ def _chunk_scan_kernels(x, dt, A, B, C, D, L: int, initial_state):
     b, S, N, P = x.shape
     bf = torch.bfloat16
     pad = (L - S % L) % L
-    x, B, C, dt = x, B.to(bf), C.to(bf), dt.float()
+    B, C, dt = B.to(bf), C.to(bf), dt.float()
     if pad:
         x, B, C = (torch.nn.functional.pad(t, (0, 0, 0, 0, 0, pad)) for t in (x, B, C))
         dt = torch.nn.functional.pad(dt, (0, 0, 0, pad))
     # rows of x: heads contiguous inside a token, one pitch from token to token over the whole batch
     ok = (x.stride(3) == 1 and x.stride(2) == P and x.stride(1) % 8 == 0 and x.data_ptr() % 16 == 0
           and (b == 1 or x.stride(0) == x.size(1) * x.stride(1)))
-    y, h = _ChunkScan.apply(x if ok else x.contiguous(), dt.contiguous(), A.float().contiguous(), B, C,
+    from ._lib import aligned
+
+    y, h = _ChunkScan.apply(x if ok else aligned(x), dt.contiguous(), A.float().contiguous(), B, C,
                             D.float().contiguous(), L, initial_state)
     return y[:, :S], h
 
