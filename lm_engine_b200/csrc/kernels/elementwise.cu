@@ -33,7 +33,7 @@ __device__ __forceinline__ void store8(__nv_bfloat16* p, const float (&f)[8]) {
 // bulk copies (one thread issues them, `stages` rows ahead), and the threads only ever wait for a row that was
 // requested `stages` rows earlier.  Rows of up to 1024 columns belong to one warp each (its own ring, no CTA barrier
 // at all), longer ones to the whole CTA (one barrier per row).
-// Measured at 8191 x 4096 (B200): residual add + norm 48.2 -> 40.4 us (268 MB, 6.6 TB/s), backward 67.5 -> 49.3 us
+// Measured at 8191 x 4096 (B200): residual add + norm 48 -> 43 us (268 MB, 6.2 TB/s), backward 67 -> 50 us
 // (268 MB, 5.4 TB/s; 63 us with two CTAs per SM instead of three).
 struct RowRing {
     int stages, row_bytes;   // row_bytes: of one operand's row
@@ -768,7 +768,7 @@ static RowPlan row_plan(int H, int nt) {
     p.ring.stages = stages;
     p.ring.row_bytes = H * 2;
     p.smem = stages * stage + groups * stages * 8;
-    // (warp rows: the weight-gradient sums of the warps, groups * H floats = 4 bytes, fit two stages of two operands)
+    // warp rows: the weight-gradient sums of the warps (groups * H floats) fit two stages of two operands
     return p;
 }
 // raises a kernel's dynamic shared memory limit once (per size it grows to), not on every launch

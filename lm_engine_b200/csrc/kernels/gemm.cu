@@ -552,11 +552,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
 // ---------------------------------------------------------------------------------------------- split contraction
 // The same product for problems whose 128 x 256 tiles cannot fill the chip (few tokens: generation steps, short
-// prompts, small fine-tuning batches).  128 x 128 tiles, two CTAs per SM, and a cluster of `splits` CTAs per tile,
-// each with a contiguous share of K: the operands of a tile stream through `splits` SMs at once, which is what bounds
-// these shapes (a single CTA waits for its ring: 0.33 us per 64-deep block of K against 0.13 us of multiplication).  Every CTA leaves its fp32 partial tile in its own shared memory
-// (the drained TMA ring), and after a cluster barrier each CTA adds the partials of its share of the rows over
-// distributed shared memory, in rank order, and runs the fused epilogue: one launch, no workspace, deterministic.
+// prompts, small fine-tuning batches): 128 x 128 tiles and a cluster of `splits` CTAs per tile, each with a contiguous
+// share of K.  The operands of a tile stream through `splits` SMs at once, which is what bounds these shapes: a single
+// CTA waits for its ring, 0.33 us per 64-deep block of K against 0.13 us of multiplication.  The ring is six stages deep
+// while there is at most one CTA per SM, three with two per SM.  Every CTA leaves its fp32 partial tile in its own
+// shared memory (the drained ring), and after a cluster barrier each CTA adds the partials of its share of the rows
+// over distributed shared memory, in rank order, and runs the fused epilogue: one launch, no workspace, deterministic.
 // Times of both kernels and the choice between them: gemm_splits() below.
 static constexpr int SK_BN = 128;
 static constexpr int SK_MAX_SPLITS = 4;
