@@ -102,7 +102,7 @@ class _SiLUMul(torch.autograd.Function):
 
 
 def silu_mul(y: torch.Tensor, gate: torch.Tensor) -> torch.Tensor:
-    """``y * silu(gate)`` (fp32 inside, one rounding); ``gate`` may be a slice of wider rows."""
+    """``y * silu(gate)``, the activation rounded to its input type; ``gate`` may be a slice of wider rows."""
     if (y.is_cuda and gate.is_cuda and y.dtype == gate.dtype == torch.bfloat16 and y.shape == gate.shape
             and y.dim() >= 2 and y.size(-1) % 8 == 0 and y.numel() > 0):
         rows = gate.stride(-1) == 1 and gate.stride(-2) % 8 == 0 and gate.data_ptr() % 16 == 0

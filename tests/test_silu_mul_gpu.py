@@ -19,6 +19,6 @@ def test_silu_mul(shape, extra):
     y64, w64 = (t.detach().double().requires_grad_(True) for t in (y, wide))
     want = y64 * torch.nn.functional.silu(w64[..., extra:])
     ref = torch.autograd.grad(want, (y64, w64), dout.double())
-    # fp32 arithmetic, one rounding of each result to bf16
+    # two roundings to bf16 (of the activation or its gradient, and of the result), each at most 2^-8 of a value
     for a, b in zip((out, *got), (want, *ref)):
-        assert float((a.double() - b).norm() / b.norm()) < 2.0 ** -8
+        assert float((a.double() - b).norm() / b.norm()) < 2.0 ** -7
