@@ -75,13 +75,33 @@ def swiglu_backward(preact: torch.Tensor, dy: torch.Tensor, tile_group: torch.Te
     return out.to(preact.dtype)
 
 
+def _row_pitch(t: torch.Tensor) -> int | None:
+    """Elements from row to row of ``t`` read as ``[rows, t.size(-1)]`` in place (16-byte accesses), ``None`` where no
+    single pitch does it.  Dimensions of size 1 have no say: their strides are arbitrary, also in tensors that count as
+    contiguous."""
+    if t.stride(-1) != 1 or t.data_ptr() % 16:
+        return None
+    pitch = following = None
+    for d in range(t.dim() - 2, -1, -1):
+        if t.size(d) == 1:
+            continue
+        if pitch is None:
+            pitch = t.stride(d)
+        elif t.stride(d) != following:
+            return None
+        following = t.stride(d) * t.size(d)
+    if pitch is None:
+        return t.size(-1)
+    return pitch if pitch % 8 == 0 and pitch >= t.size(-1) else None
+
+
 class _SiLUMul(torch.autograd.Function):
     @staticmethod
     def forward(ctx, y, gate):
         I = y.size(-1)
         y2 = _lib.aligned(y.reshape(-1, I))
         out = torch.empty_like(y2)
-        _lib.check(_lib.cuda_lib().lme_silu_mul_fwd(y2.data_ptr(), gate.data_ptr(), gate.stride(-2), out.data_ptr(),
+        _lib.check(_lib.cuda_lib().lme_silu_mul_fwd(y2.data_ptr(), gate.data_ptr(), _row_pitch(gate), out.data_ptr(),
                                                     y2.size(0), I, _lib.stream_ptr()), "lme_silu_mul_fwd")
         _lib.count_launch()
         ctx.save_for_backward(y2, gate)
@@ -91,23 +111,25 @@ class _SiLUMul(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dout):
         y2, gate = ctx.saved_tensors
+        if _row_pitch(gate) is None:        # a saved-tensor hook may return other strides
+            gate = _lib.aligned(gate)
         T, I = y2.shape
         d2 = _lib.aligned(dout.reshape(T, I))
         dy, dg = torch.empty_like(y2), torch.empty_like(y2)
-        _lib.check(_lib.cuda_lib().lme_silu_mul_bwd(d2.data_ptr(), y2.data_ptr(), gate.data_ptr(), gate.stride(-2),
+        _lib.check(_lib.cuda_lib().lme_silu_mul_bwd(d2.data_ptr(), y2.data_ptr(), gate.data_ptr(), _row_pitch(gate),
                                                     dy.data_ptr(), dg.data_ptr(), T, I, _lib.stream_ptr()),
                    "lme_silu_mul_bwd")
         _lib.count_launch()
         return dy.view(ctx.shape), dg.view(gate.shape)
 
 
+def _silu_mul_kernel_usable(y: torch.Tensor, gate: torch.Tensor) -> bool:
+    return (y.is_cuda and gate.is_cuda and y.dtype == gate.dtype == torch.bfloat16 and y.shape == gate.shape
+            and y.dim() >= 2 and y.size(-1) % 8 == 0 and y.numel() > 0)
+
+
 def silu_mul(y: torch.Tensor, gate: torch.Tensor) -> torch.Tensor:
     """``y * silu(gate)``, the activation rounded to its input type; ``gate`` may be a slice of wider rows."""
-    if (y.is_cuda and gate.is_cuda and y.dtype == gate.dtype == torch.bfloat16 and y.shape == gate.shape
-            and y.dim() >= 2 and y.size(-1) % 8 == 0 and y.numel() > 0):
-        rows = gate.stride(-1) == 1 and gate.stride(-2) % 8 == 0 and gate.data_ptr() % 16 == 0
-        pitch = gate.stride(-2)
-        for d in range(gate.dim() - 2, 0, -1):       # one pitch from row to row through the leading dimensions
-            rows = rows and (gate.size(d - 1) == 1 or gate.stride(d - 1) == gate.size(d) * gate.stride(d))
-        return _SiLUMul.apply(y, gate if rows and pitch >= gate.size(-1) else _lib.aligned(gate))
+    if _silu_mul_kernel_usable(y, gate):
+        return _SiLUMul.apply(y, gate if _row_pitch(gate) is not None else _lib.aligned(gate))
     return y * torch.nn.functional.silu(gate.float()).to(gate.dtype)

@@ -1,0 +1,72 @@
+"""Addresses that the wrappers hand to the kernels, with the library replaced by a recorder: what a kernel would read
+has to lie inside the operand's storage, also where dimensions of size 1 carry strides of their own (contiguous() and
+clone() keep those)."""
+
+import pytest
+import torch
+
+from lm_engine_b200.ops import _lib
+
+BF = torch.bfloat16
+
+
+class _Recorder:
+    def __init__(self):
+        self.calls = {}
+
+    def __getattr__(self, name):
+        def call(*args):
+            self.calls[name] = args
+            return 0
+        return call
+
+
+@pytest.fixture
+def lib(monkeypatch):
+    rec = _Recorder()
+    monkeypatch.setattr(_lib, "cuda_lib", lambda: rec)
+    monkeypatch.setattr(_lib, "stream_ptr", lambda: 0)
+    return rec
+
+
+def _wide(B, S, W, offset, C):
+    """Slice ``[B, S, C]`` of a projection's rows of W elements, that start at `offset`."""
+    return torch.zeros(B, S, W, dtype=BF)[..., offset:offset + C]
+
+
+GATES = {
+    # (gate, rows the kernel may read in place at this pitch; None: a copy)
+    "one row, odd width": (lambda: _wide(1, 1, 1542, 6, 1536), None),
+    "one row, odd width, aligned": (lambda: _wide(1, 1, 1544 + 3, 8, 1536), 1536),
+    "batch, one step": (lambda: _wide(5, 1, 528, 16, 512), 528),
+    "rows of a batch": (lambda: _wide(2, 7, 528, 16, 512), 528),
+    "odd width": (lambda: _wide(2, 7, 521, 8, 512), None),
+    "transposed unit dimension": (lambda: torch.zeros(7, 64, dtype=BF)[None].transpose(0, 1), 64),
+    "permuted": (lambda: torch.zeros(3, 5, 64, dtype=BF).transpose(0, 1), None),
+    "expanded": (lambda: torch.zeros(1, 64, dtype=BF).expand(4, 64), None),
+}
+
+
+@pytest.mark.parametrize("name", GATES)
+def test_gate_rows(lib, monkeypatch, name):
+    from lm_engine_b200.ops import activation
+
+    monkeypatch.setattr(activation, "_silu_mul_kernel_usable", lambda y, gate: True)
+    make, in_place = GATES[name]
+    gate = make().requires_grad_(True)
+    y = torch.zeros(gate.shape, dtype=BF, requires_grad=True)
+    read = {}
+    out = activation.silu_mul(y, gate)
+    read["fwd"] = lib.calls["lme_silu_mul_fwd"][1:3]
+    out.backward(torch.zeros_like(out))
+    read["bwd"] = lib.calls["lme_silu_mul_bwd"][2:4]
+    assert y.grad.shape == y.shape and gate.grad.shape == gate.shape
+    I, T = gate.size(-1), gate.numel() // gate.size(-1)
+    base, n = gate.untyped_storage().data_ptr(), gate.untyped_storage().nbytes() // 2
+    for ptr, pitch in read.values():
+        assert ptr % 16 == 0 and pitch % 8 == 0
+        if in_place is None:
+            assert pitch == I        # a dense copy
+        else:
+            assert pitch == in_place and ptr == gate.data_ptr()
+            assert 0 <= (ptr - base) // 2 and (ptr - base) // 2 + (T - 1) * pitch + I <= n
