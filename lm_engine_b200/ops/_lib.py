@@ -165,8 +165,19 @@ def ptr(t: torch.Tensor | None) -> int | None:
     return None if t is None else t.data_ptr()
 
 
+def strides(t: torch.Tensor) -> tuple[int, ...]:
+    """Element strides of ``t``, those of size-1 dimensions as in a dense tensor: PyTorch leaves them arbitrary and hands
+    them through ``contiguous()`` and ``clone()``, so they say nothing about where elements are."""
+    out, dense = [], 1
+    for size, stride in zip(reversed(t.shape), reversed(t.stride())):
+        out.append(dense if size == 1 else stride)
+        dense *= size
+    return tuple(reversed(out))
+
+
 def aligned(t: torch.Tensor) -> torch.Tensor:
-    """``t`` contiguous and on a 16-byte boundary (kernels with 16-byte accesses; a contiguous view may start anywhere)."""
+    """``t`` contiguous and on a 16-byte boundary (kernels with 16-byte accesses; a contiguous view may start anywhere).
+    Its strides go to a kernel through :func:`strides`."""
     t = t.contiguous()
     return t if t.data_ptr() % 16 == 0 else t.clone()
 

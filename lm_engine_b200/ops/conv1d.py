@@ -25,6 +25,18 @@ def causal_conv1d_reference(x: torch.Tensor, weight: torch.Tensor, bias: torch.T
     return y
 
 
+def _rows(x: torch.Tensor, K: int) -> tuple[torch.Tensor, int, int]:
+    """x with its batch and time strides as the kernels take them: the four-tap kernels read a slice of wider rows in
+    place (16-byte rows), everything else is a dense copy."""
+    from . import _lib
+
+    x_b, x_t, x_c = _lib.strides(x)
+    if K != 4 or x_c != 1 or x_t % 8 or x_b % 8 or x.data_ptr() % 16:
+        x = _lib.aligned(x)
+        x_b, x_t, _ = _lib.strides(x)
+    return x, x_b, x_t
+
+
 class _CausalConv1d(torch.autograd.Function):
     """CUDA path: one pass forward (activation fused), one pass backward that recomputes the pre-activation."""
 
@@ -34,15 +46,13 @@ class _CausalConv1d(torch.autograd.Function):
 
         B, S, C = x.shape
         K = weight.size(1)
-        # the four-tap kernels read a slice of wider rows in place (aligned to 16 bytes)
-        if K != 4 or x.stride(2) != 1 or x.stride(1) % 8 or x.stride(0) % 8 or x.data_ptr() % 16:
-            x = x.contiguous()
+        x, x_b, x_t = _rows(x, K)
         w = _lib.aligned(weight)
         init = initial_state.to(x.dtype).contiguous() if initial_state is not None else None
         y = torch.empty((B, S, C), dtype=x.dtype, device=x.device)
-        _lib.check(_lib.cuda_lib().lme_causal_conv1d_fwd(x.data_ptr(), x.stride(0), x.stride(1), w.data_ptr(),
-                                                         _lib.ptr(bias), _lib.ptr(init), y.data_ptr(), B, S, C, K,
-                                                         int(silu), _lib.stream_ptr()), f"lme_causal_conv1d_fwd B={B} S={S} C={C} K={K}")
+        _lib.check(_lib.cuda_lib().lme_causal_conv1d_fwd(
+            x.data_ptr(), x_b, x_t, w.data_ptr(), _lib.ptr(bias), _lib.ptr(init), y.data_ptr(), B, S, C, K, int(silu),
+            _lib.stream_ptr()), f"lme_causal_conv1d_fwd B={B} S={S} C={C} K={K}")
         _lib.count_launch()
         ctx.save_for_backward(x, w, bias, init)
         ctx.silu = silu
@@ -55,15 +65,16 @@ class _CausalConv1d(torch.autograd.Function):
         x, w, bias, init = ctx.saved_tensors
         B, S, C = x.shape
         K = w.size(1)
-        dy = dy.contiguous()
+        x, x_b, x_t = _rows(x, K)           # a saved-tensor hook may return other strides
+        dy = _lib.aligned(dy)
         dx = torch.empty((B, S, C), dtype=x.dtype, device=x.device)
         dw = torch.zeros((C, K), dtype=torch.float32, device=x.device)
         db = torch.zeros(C, dtype=torch.float32, device=x.device) if bias is not None else None
         dinit = (torch.empty((B, C, K - 1), dtype=torch.float32, device=x.device)
                  if init is not None and ctx.needs_input_grad[3] else None)
         _lib.check(_lib.cuda_lib().lme_causal_conv1d_bwd(
-            x.data_ptr(), x.stride(0), x.stride(1), w.data_ptr(), _lib.ptr(bias), _lib.ptr(init), dy.data_ptr(), dx.data_ptr(), dw.data_ptr(),
-            _lib.ptr(db), _lib.ptr(dinit), B, S, C, K, int(ctx.silu), _lib.stream_ptr()),
+            x.data_ptr(), x_b, x_t, w.data_ptr(), _lib.ptr(bias), _lib.ptr(init), dy.data_ptr(), dx.data_ptr(),
+            dw.data_ptr(), _lib.ptr(db), _lib.ptr(dinit), B, S, C, K, int(ctx.silu), _lib.stream_ptr()),
             f"lme_causal_conv1d_bwd B={B} S={S} C={C} K={K}")
         _lib.count_launch()
         return (dx, dw.to(w.dtype), db.to(bias.dtype) if db is not None else None,

@@ -70,3 +70,36 @@ def test_gate_rows(lib, monkeypatch, name):
         else:
             assert pitch == in_place and ptr == gate.data_ptr()
             assert 0 <= (ptr - base) // 2 and (ptr - base) // 2 + (T - 1) * pitch + I <= n
+
+
+ROWS = {
+    # x [B, S, C], element strides (batch, time) of an in-place read at four taps; None: a dense copy
+    "one row, odd width": (lambda: _wide(1, 1, 1001, 8, 16), (16, 16)),
+    "one row, aligned width": (lambda: _wide(1, 1, 1008, 8, 16), (16, 16)),
+    "one row, misaligned": (lambda: _wide(1, 1, 1008, 4, 16), None),
+    "batch, one step": (lambda: _wide(3, 1, 1008, 8, 16), (1008, 16)),
+    "batch, one step, odd width": (lambda: _wide(3, 1, 1001, 8, 16), None),
+    "steps": (lambda: _wide(2, 5, 48, 8, 16), (240, 48)),
+    "unit batch of odd stride": (lambda: torch.zeros(5 * 16 + 3, dtype=BF).as_strided((1, 5, 16), (83, 16, 1)), (80, 16)),
+    "dense, misaligned": (lambda: torch.zeros(2 * 5 * 16 + 1, dtype=BF)[1:].view(2, 5, 16), None),
+}
+
+
+@pytest.mark.parametrize("K", [3, 4, 6])
+@pytest.mark.parametrize("name", ROWS)
+def test_convolution_rows(lib, name, K):
+    from lm_engine_b200.ops.conv1d import _CausalConv1d
+
+    make, in_place = ROWS[name]
+    x = make().requires_grad_(True)
+    B, S, C = x.shape
+    y = _CausalConv1d.apply(x, torch.zeros(C, K, dtype=BF, requires_grad=True), None, None, True)
+    dy = torch.zeros(y.numel() + 1, dtype=BF)[1:].view(y.shape)          # a contiguous gradient may start anywhere
+    y.backward(dy)
+    for ptr, x_b, x_t in (lib.calls["lme_causal_conv1d_fwd"][:3], lib.calls["lme_causal_conv1d_bwd"][:3]):
+        assert ptr % 16 == 0
+        if K == 4 and in_place is not None:
+            assert (x_b, x_t) == in_place and ptr == x.data_ptr()
+        else:
+            assert (x_b, x_t) == (S * C, C)
+    assert lib.calls["lme_causal_conv1d_bwd"][6] % 16 == 0

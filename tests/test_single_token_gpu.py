@@ -18,7 +18,17 @@ def _gated_deltanet(heads):
                          0, "normal", 0.05, None, 4, False)
 
 
-MIXERS = {"gated-deltanet-1": lambda: _gated_deltanet(1), "gated-deltanet-3": lambda: _gated_deltanet(3),
+def _mamba2(heads, taps):
+    from lm_engine_b200.models.config import Mamba2Args
+    from lm_engine_b200.models.layers.mamba2 import Mamba2
+
+    return Mamba2(256, Mamba2Args(state_size=16, intermediate_size=32 * heads, num_heads=heads, conv_kernel_size=taps,
+                                  activation_function="silu", num_groups=1, chunk_size=32,
+                                  normalization_function="rmsnorm"), 1e-5, 0.05, None, "normal", 4, 0)
+
+
+MIXERS = {"mamba2-4": lambda: _mamba2(4, 4), "mamba2-3-three-taps": lambda: _mamba2(3, 3),
+          "mamba2-8-three-taps": lambda: _mamba2(8, 3), "gated-deltanet-1": lambda: _gated_deltanet(1), "gated-deltanet-3": lambda: _gated_deltanet(3),
           "gated-deltanet-4": lambda: _gated_deltanet(4)}
 
 
@@ -60,3 +70,21 @@ def test_gate_of_single_rows(make):
     # two roundings to bf16, each at most 2^-8 of a value
     for a, b in zip((out.detach(), *got), (want.detach(), *torch.autograd.grad(want, (y64, w64), dout.double()))):
         assert float((a.double() - b).norm() / b.norm()) < 2.0 ** -7
+
+
+@pytest.mark.parametrize("K", [3, 4])
+@pytest.mark.parametrize("width,offset", [(1001, 8), (1008, 8), (1008, 4)])
+def test_convolution_of_a_single_row(width, offset, K):
+    from lm_engine_b200.ops.conv1d import causal_conv1d, causal_conv1d_reference
+
+    wide = torch.randn(1, 1, width, device="cuda").to(BF).requires_grad_(True)
+    w = torch.randn(64, K, device="cuda").to(BF).requires_grad_(True)
+    state = torch.randn(1, 64, K - 1, device="cuda").to(BF).requires_grad_(True)
+    y = causal_conv1d(wide[..., offset:offset + 64], w, None, state, "silu")
+    dy = torch.randn(y.numel() + 1, device="cuda").to(BF)[1:].view(y.shape)
+    ins = [t.detach().double().requires_grad_(True) for t in (wide, w, state)]
+    want = causal_conv1d_reference(ins[0][..., offset:offset + 64], ins[1], None, ins[2], "silu")
+    ref = torch.autograd.grad(want, ins, dy.double())
+    # fp32 arithmetic, one rounding of each result to bf16
+    for a, b in zip((y.detach(), *torch.autograd.grad(y, (wide, w, state), dy)), (want.detach(), *ref)):
+        assert float((a.double() - b).norm() / b.norm()) < 2.0 ** -8
