@@ -292,6 +292,7 @@ class _GatedDeltaBlocks(torch.autograd.Function):
         from .gemm import _bmm_kernel
 
         q, k, v, g, beta, wk, qe, ke, qk, a, x, u_all, h_all = ctx.saved_tensors
+        q, k, v = (_delta_operand(t) for t in (q, k, v))         # a saved-tensor hook may return other strides
         scale, use_qk_l2norm, has_h0 = ctx.cfg
         B, S, N, K = q.shape
         V, L = v.size(-1), CHUNK
@@ -332,15 +333,18 @@ class _GatedDeltaBlocks(torch.autograd.Function):
 
 def _delta_strides(*tensors):
     """Batch, token and head strides of ``[B, S, N, X]`` tensors as a C array."""
-    flat = [t.stride(d) for t in tensors for d in range(3)]
+    from ._lib import strides
+
+    flat = [s for t in tensors for s in strides(t)[:3]]
     return (ctypes.c_longlong * len(flat))(*flat)
 
 
 def _delta_operand(t: torch.Tensor) -> torch.Tensor:
     """Rows that the kernels read in 16-byte pieces (any batch / token / head pitch that keeps them aligned)."""
-    from ._lib import aligned
+    from ._lib import aligned, strides
 
-    ok = t.stride(3) == 1 and t.data_ptr() % 16 == 0 and not any(t.stride(d) % 8 for d in range(3))
+    *pitches, inner = strides(t)
+    ok = inner == 1 and t.data_ptr() % 16 == 0 and not any(p % 8 for p in pitches)
     return t if ok else aligned(t)
 
 

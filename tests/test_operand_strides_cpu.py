@@ -103,3 +103,18 @@ def test_convolution_rows(lib, name, K):
         else:
             assert (x_b, x_t) == (S * C, C)
     assert lib.calls["lme_causal_conv1d_bwd"][6] % 16 == 0
+
+
+@pytest.mark.parametrize("shape,stride,in_place", [
+    ((1, 9, 2, 128), (9 * 256 + 3, 256, 128), True), ((2, 9, 1, 128), (9 * 144, 144, 77), True),
+    ((1, 9, 1, 128), (5, 128, 3), True), ((2, 9, 2, 128), (9 * 262, 262, 128), False),
+    ((1, 9, 2, 128), (0, 262, 128), False), ((2, 9, 2, 128), (9 * 288, 288, 128), True)])
+def test_delta_rule_operands(shape, stride, in_place):
+    from lm_engine_b200.ops.recurrence import _delta_operand, _delta_strides
+
+    t = torch.zeros(2 * 9 * 512, dtype=BF).as_strided(shape, (*stride, 1))
+    u = _delta_operand(t)
+    assert (u.data_ptr() == t.data_ptr()) == in_place
+    got = tuple(_delta_strides(u))
+    dense = (9 * shape[2] * 128, shape[2] * 128, 128)
+    assert got == tuple((s if in_place and n > 1 else d) for s, n, d in zip(stride, shape, dense))
