@@ -94,7 +94,10 @@ struct RowGroup {
     }
     __device__ __forceinline__ float sum(float v, int it) {
         v = warp_sum(v);
-        if (WARP) return v;
+        if (WARP) {
+            __syncwarp();   // shuffles order no memory: every lane has read its stage before lane 0 refills it
+            return v;
+        }
         float* buf = red + (it & 1) * 32;
         if ((threadIdx.x & 31) == 0) buf[threadIdx.x >> 5] = v;
         __syncthreads();
