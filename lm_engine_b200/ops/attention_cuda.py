@@ -70,10 +70,12 @@ def decode_attention(q, k, v, *, softmax_scale: float, sliding_window: int | Non
     position, so causality hides nothing; ``sliding_window`` keeps the last that many keys.  Rows that attend to
     nothing are zero; values of hidden keys are not read into the sum."""
     def rows(t):
-        ok = t.stride(3) == 1 and t.data_ptr() % 16 == 0 and not any(t.stride(d) % 8 for d in range(3))
+        *pitches, inner = _lib.strides(t)
+        ok = inner == 1 and t.data_ptr() % 16 == 0 and not any(p % 8 for p in pitches)
         return t if ok else _lib.aligned(t)
 
     q, k, v = rows(q), rows(k), rows(v)
+    (q_b, _, q_h, _), (k_b, k_s, k_h, _), (v_b, v_s, v_h, _) = (_lib.strides(t) for t in (q, k, v))
     B, _, Hq, D = q.shape
     Sk, Hkv = k.size(1), k.size(2)
     out = torch.empty((B, 1, Hq, D), dtype=q.dtype, device=q.device)
@@ -82,9 +84,8 @@ def decode_attention(q, k, v, *, softmax_scale: float, sliding_window: int | Non
         mask = attention_mask.bool().contiguous()
     window = Sk if sliding_window is None else min(sliding_window, Sk)
     _lib.check(_lib.cuda_lib().lme_decode_attention(
-        q.data_ptr(), q.stride(0), q.stride(2), k.data_ptr(), k.stride(0), k.stride(1), k.stride(2), v.data_ptr(),
-        v.stride(0), v.stride(1), v.stride(2), _lib.ptr(mask), Sk, out.data_ptr(), B, Sk, Hkv, Hq // Hkv, D, window,
-        softmax_scale, _lib.stream_ptr()), f"lme_decode_attention B={B} Sk={Sk} Hq={Hq} Hkv={Hkv} D={D}")
+        q.data_ptr(), q_b, q_h, k.data_ptr(), k_b, k_s, k_h, v.data_ptr(), v_b, v_s, v_h, _lib.ptr(mask), Sk,
+        out.data_ptr(), B, Sk, Hkv, Hq // Hkv, D, window, softmax_scale, _lib.stream_ptr()), f"lme_decode_attention B={B} Sk={Sk} Hq={Hq} Hkv={Hkv} D={D}")
     _lib.count_launch()
     return out
 

@@ -118,3 +118,17 @@ def test_delta_rule_operands(shape, stride, in_place):
     got = tuple(_delta_strides(u))
     dense = (9 * shape[2] * 128, shape[2] * 128, 128)
     assert got == tuple((s if in_place and n > 1 else d) for s, n, d in zip(stride, shape, dense))
+
+
+def test_one_token_attention_operands(lib):
+    from lm_engine_b200.ops.attention_cuda import decode_attention
+
+    flat = torch.zeros(4096, dtype=BF)
+    q = flat.as_strided((1, 1, 4, 64), (1003, 77, 64, 1))          # a unit batch of any stride
+    k = flat.as_strided((1, 6, 1, 64), (5, 72, 3, 1))              # and a single head
+    v = flat.as_strided((1, 6, 1, 64), (5, 70, 3, 1))              # rows between 16-byte boundaries: a copy
+    decode_attention(q, k, v, softmax_scale=1.0)
+    args = lib.calls["lme_decode_attention"]
+    assert args[:3] == (flat.data_ptr(), 256, 64)
+    assert args[3:7] == (flat.data_ptr(), 384, 72, 64)
+    assert args[7] != flat.data_ptr() and args[8:11] == (384, 64, 64)
