@@ -140,6 +140,11 @@ def scan_glue_eligible(x: torch.Tensor, L: int, Sd: int) -> bool:
             and Sd % 8 == 0 and 0 < b * N <= 65535 and 0 < b * ((S + L - 1) // L) <= 65535 and FUSED_INTRA_CHUNK)
 
 
+def _per_head(t: torch.Tensor, N: int) -> bool:
+    """One value per head, or one for all; other shapes that broadcast take the general path."""
+    return t.numel() in (1, N) and t.shape[-1:].numel() == t.numel()
+
+
 def _intra_chunk_fused(Cc, Bc, ct, xdt):
     """CUDA path of the intra-chunk term.  Cc / Bc ``[b, nc, L, G, Sd]``, ct ``[b, nc, N, L]`` fp32,
     xdt ``[b, nc, L, N, P]`` fp32 -> ``[b, nc, L, N, P]`` fp32."""
@@ -162,7 +167,7 @@ def ssd_chunk_scan(x, dt, A, B, C, D, chunk_size: int, initial_state=None):
     dtype = x.dtype
     L = chunk_size
     pad = (L - S % L) % L
-    if scan_glue_eligible(x, L, Sd):
+    if scan_glue_eligible(x, L, Sd) and _per_head(A, N) and _per_head(D, N):
         return _chunk_scan_kernels(x, dt, A, B, C, D, L, initial_state)
     xf, dtf, Bf, Cf = x.float(), dt.float(), B.float(), C.float()
     if pad:
@@ -343,21 +348,28 @@ def _chunk_rows(t: torch.Tensor, bc: int, L: int) -> torch.Tensor:
 
 
 def _chunk_scan_kernels(x, dt, A, B, C, D, L: int, initial_state):
-    """Pads to whole chunks (padded steps have dt = 0: decay 1, no input) and runs :class:`_ChunkScan`."""
+    """Pads to whole chunks (padded steps have dt = 0: decay 1, no input) and runs :class:`_ChunkScan`.  The kernels
+    get bare addresses, so every operand takes its full shape here (a mismatch raises)."""
     b, S, N, P = x.shape
+    G, Sd = B.shape[-2:]
+    if N % G:
+        raise ValueError(f"ssd: {N} heads do not split into {G} groups")
     bf = torch.bfloat16
     pad = (L - S % L) % L
     B, C, dt = B.to(bf), C.to(bf), dt.float()
     if pad:
         x, B, C = (torch.nn.functional.pad(t, (0, 0, 0, 0, 0, pad)) for t in (x, B, C))
         dt = torch.nn.functional.pad(dt, (0, 0, 0, pad))
+    B, C, dt = B.reshape(b, S + pad, G, Sd), C.reshape(b, S + pad, G, Sd), dt.reshape(b, S + pad, N)
+    A, D = (t.float().reshape(-1).expand(N).contiguous() for t in (A, D))
+    if initial_state is not None:
+        initial_state = initial_state.expand(b, N, P, Sd)
     # rows of x: heads contiguous inside a token, one pitch from token to token over the whole batch
     ok = (x.stride(3) == 1 and x.stride(2) == P and x.stride(1) % 8 == 0 and x.data_ptr() % 16 == 0
           and (b == 1 or x.stride(0) == x.size(1) * x.stride(1)))
     from ._lib import aligned
 
-    y, h = _ChunkScan.apply(x if ok else aligned(x), dt.contiguous(), A.float().contiguous(), B, C,
-                            D.float().contiguous(), L, initial_state)
+    y, h = _ChunkScan.apply(x if ok else aligned(x), dt.contiguous(), A, B, C, D, L, initial_state)
     return y[:, :S], h
 
 

@@ -1,0 +1,39 @@
+"""One decay, skip weight or initial state for all heads or sequences in the SSD scan's kernels."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def test_shared_decay_skip_and_state():
+    from lm_engine_b200.ops.ssd import ssd_chunk_scan
+
+    b, S, N, P, G, Sd = 2, 70, 4, 32, 2, 16
+    g = torch.Generator(device="cuda").manual_seed(0)
+
+    def r(*s):
+        return torch.randn(*s, generator=g, device="cuda")
+
+    x, B, C = (r(*s).to(torch.bfloat16) for s in ((b, S, N, P), (b, S, G, Sd), (b, S, G, Sd)))
+    dt = torch.rand(b, S, N, generator=g, device="cuda")
+    shared = [(-r(1).abs()).requires_grad_(True), r(1).requires_grad_(True), r(1, N, P, Sd).requires_grad_(True)]
+    full = [t.detach().expand(s).clone().requires_grad_(True) for t, s in zip(shared, ((N,), (N,), (b, N, P, Sd)))]
+    dy, dh, outs = r(b, S, N, P).to(torch.bfloat16), r(b, N, P, Sd), []
+    for A, D, h0 in (shared, full):
+        y, h = ssd_chunk_scan(x, dt, A, B, C, D, 32, initial_state=h0)
+        outs.append((y, h, *torch.autograd.grad((y, h), (A, D, h0), (dy, dh))))
+    a, f = outs
+    assert torch.equal(a[0], f[0]) and torch.equal(a[1], f[1])
+    # the same fp32 gradients, added over heads or sequences in any order
+    for got, want, dim in zip(a[2:], f[2:], (0, 0, 0)):
+        torch.testing.assert_close(got, want.sum(dim, keepdim=True), rtol=1e-5, atol=1e-4 * float(want.abs().max()))
+
+
+def test_a_step_width_that_does_not_fit_raises():
+    from lm_engine_b200.ops.ssd import ssd_chunk_scan
+
+    x, B = torch.zeros(1, 32, 4, 32, device="cuda", dtype=torch.bfloat16), torch.zeros(1, 32, 1, 16, device="cuda")
+    with pytest.raises(RuntimeError):
+        ssd_chunk_scan(x, torch.zeros(1, 32, 1, device="cuda"), -torch.ones(4, device="cuda"), B, B,
+                       torch.ones(4, device="cuda"), 32)
