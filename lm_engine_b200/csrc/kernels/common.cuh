@@ -10,6 +10,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <type_traits>
 
 #ifndef LME_WAIT_LIMIT_NS
 #define LME_WAIT_LIMIT_NS 2000000000ull  // 2 s

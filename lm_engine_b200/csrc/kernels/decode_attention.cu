@@ -43,6 +43,10 @@ __device__ __forceinline__ uint4 ld_stream(const __nv_bfloat16* p) {
     return r;
 }
 __device__ __forceinline__ uint32_t word(const uint4& u, int i) { return i == 0 ? u.x : i == 1 ? u.y : i == 2 ? u.z : u.w; }
+// 0xffff in the halves of a bf16 pair that are infinite or not a number
+__device__ __forceinline__ uint32_t not_finite(uint32_t w) {
+    return ((w & 0x7f80u) == 0x7f80u ? 0xffffu : 0u) | ((w & 0x7f800000u) == 0x7f800000u ? 0xffff0000u : 0u);
+}
 __device__ __forceinline__ float ld_cluster(const float* p, uint32_t cta) {
     uint32_t a;
     float v;
@@ -54,17 +58,20 @@ __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 template <int D>
-__global__ void __launch_bounds__(WARPS * 32, 3) decode_attention_kernel(const Args p) {
+struct Partials {          // of the warps
+    float acc[WARPS][8][D];
+    float m[WARPS][8], l[WARPS][8];
+};
+
+// One warp's share of the keys [k0, k1); returns whether any of its sums is not finite.
+// An infinite value times the zero or negative lower terms of its weight is not the infinity that it should be, so a
+// warp with such a sum goes over its keys a second time, out of line, where values that are not finite meet the
+// leading term alone (!FINITE).
+template <int D, bool FINITE>
+__device__ __forceinline__ bool attend_keys(const Args& p, Partials<D>& s, int kvh, int hb, long long b, int heads, int k0,
+                                            int k1) {
     constexpr int KC = D / 32;    // 16-byte pieces of a key per lane
     constexpr int VC = D / 64;    // 16-byte pieces of a value row per lane
-    __shared__ float s_acc[WARPS][8][D];
-    __shared__ float s_m[WARPS][8], s_l[WARPS][8];
-    __shared__ float c_acc[8][D];
-    __shared__ float c_m[8], c_l[8];
-    const int splits = gridDim.x, split = blockIdx.x;
-    const int kvh = blockIdx.y / p.head_blocks, hb = blockIdx.y % p.head_blocks;
-    const long long b = blockIdx.z;
-    const int heads = min(8, p.G - hb * 8);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
 
     // query fragments; rows >= heads are zero
@@ -84,10 +91,6 @@ __global__ void __launch_bounds__(WARPS * 32, 3) decode_attention_kernel(const A
     const __nv_bfloat16* kb = p.k + b * p.k_b + static_cast<long long>(kvh) * p.k_h + 8 * t;
     const __nv_bfloat16* vb = p.v + b * p.v_b + static_cast<long long>(kvh) * p.v_h + 8 * g;
     const unsigned char* mb = p.mask != nullptr ? p.mask + b * p.mask_b : nullptr;
-
-    const int n = p.Sk - p.first;
-    const int per = ((n + splits - 1) / splits + 15) & ~15;
-    const int k0 = p.first + min(n, split * per), k1 = p.first + min(n, (split + 1) * per);
 
     float acc[D / 8][4];
 #pragma unroll
@@ -127,22 +130,22 @@ __global__ void __launch_bounds__(WARPS * 32, 3) decode_attention_kernel(const A
         load_values(k0 + warp * 16);
     }
     for (int base = k0 + warp * 16; base < k1; base += STEP) {
-        float s[2][4];
+        float sc[2][4];
 #pragma unroll
         for (int tile = 0; tile < 2; ++tile) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) s[tile][i] = 0.f;
+            for (int i = 0; i < 4; ++i) sc[tile][i] = 0.f;
 #pragma unroll
             for (int ks = 0; ks < D / 16; ++ks) {
                 const uint32_t a[4] = {qa[ks][0], 0u, qa[ks][1], 0u};
-                mma16816(s[tile], a, word(kw[tile][ks >> 1], 2 * (ks & 1)), word(kw[tile][ks >> 1], 2 * (ks & 1) + 1));
+                mma16816(sc[tile], a, word(kw[tile][ks >> 1], 2 * (ks & 1)), word(kw[tile][ks >> 1], 2 * (ks & 1) + 1));
             }
         }
         if (base + STEP < k1) load_keys(base + STEP);
         float x[4], mx = m;
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            x[e] = (ok >> e & 1) ? s[e >> 1][e & 1] * p.scale : -INFINITY;
+            x[e] = (ok >> e & 1) ? sc[e >> 1][e & 1] * p.scale : -INFINITY;
             mx = fmaxf(mx, x[e]);
         }
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
@@ -170,8 +173,14 @@ __global__ void __launch_bounds__(WARPS * 32, 3) decode_attention_kernel(const A
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 const uint32_t sel = (i & 1) ? 0x7632u : 0x5410u;
-                const uint32_t b0 = __byte_perm(word(vw[0][j], i >> 1), word(vw[1][j], i >> 1), sel);
-                const uint32_t b1 = __byte_perm(word(vw[2][j], i >> 1), word(vw[3][j], i >> 1), sel);
+                uint32_t b0 = __byte_perm(word(vw[0][j], i >> 1), word(vw[1][j], i >> 1), sel);
+                uint32_t b1 = __byte_perm(word(vw[2][j], i >> 1), word(vw[3][j], i >> 1), sel);
+                if (!FINITE) {
+                    const uint32_t ah[4] = {hi[0], hi[0], hi[1], hi[1]}, n0 = not_finite(b0), n1 = not_finite(b1);
+                    mma16816(acc[j * 8 + i], ah, b0 & n0, b1 & n1);
+                    b0 &= ~n0;
+                    b1 &= ~n1;
+                }
                 mma16816(acc[j * 8 + i], a0, b0, b1);
                 mma16816(acc[j * 8 + i], a1, b0, b1);
             }
@@ -180,30 +189,55 @@ __global__ void __launch_bounds__(WARPS * 32, 3) decode_attention_kernel(const A
     l += __shfl_xor_sync(0xffffffffu, l, 1);
     l += __shfl_xor_sync(0xffffffffu, l, 2);
     // accumulator i of piece j: columns 2t, 2t + 1 of the product are dims 64 j + 8 (2t) + i and 64 j + 8 (2t + 1) + i
+    float zero = 0.f;
 #pragma unroll
     for (int j = 0; j < VC; ++j)
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const float* a = acc[j * 8 + i];
-            s_acc[warp][g][64 * j + 16 * t + i] = a[0] + a[2];
-            s_acc[warp][g][64 * j + 16 * t + 8 + i] = a[1] + a[3];
+            const float c0 = a[0] + a[2], c1 = a[1] + a[3];
+            s.acc[warp][g][64 * j + 16 * t + i] = c0;
+            s.acc[warp][g][64 * j + 16 * t + 8 + i] = c1;
+            zero += (c0 + c1) * 0.f;
         }
     if (t == 0) {
-        s_m[warp][g] = m;
-        s_l[warp][g] = l;
+        s.m[warp][g] = m;
+        s.l[warp][g] = l;
     }
+    return __any_sync(0xffffffffu, zero != 0.f);
+}
+template <int D>
+__device__ __noinline__ void attend_keys_not_finite(const Args& p, Partials<D>& s, int kvh, int hb, long long b, int heads,
+                                                    int k0, int k1) {
+    attend_keys<D, false>(p, s, kvh, hb, b, heads, k0, k1);
+}
+
+template <int D>
+__global__ void __launch_bounds__(WARPS * 32, 3) decode_attention_kernel(const __grid_constant__ Args p) {
+    __shared__ Partials<D> part;
+    __shared__ float c_acc[8][D];
+    __shared__ float c_m[8], c_l[8];
+    const int splits = gridDim.x, split = blockIdx.x;
+    const int kvh = blockIdx.y / p.head_blocks, hb = blockIdx.y % p.head_blocks;
+    const long long b = blockIdx.z;
+    const int heads = min(8, p.G - hb * 8);
+    const int n = p.Sk - p.first;
+    const int per = ((n + splits - 1) / splits + 15) & ~15;
+    const int k0 = p.first + min(n, split * per), k1 = p.first + min(n, (split + 1) * per);
+    if (attend_keys<D, true>(p, part, kvh, hb, b, heads, k0, k1))
+        attend_keys_not_finite<D>(p, part, kvh, hb, b, heads, k0, k1);
     __syncthreads();
     for (int u = threadIdx.x; u < heads * D; u += WARPS * 32) {
         const int r = u / D, d = u % D;
         float M = -INFINITY;
 #pragma unroll
-        for (int w = 0; w < WARPS; ++w) M = fmaxf(M, s_m[w][r]);
+        for (int w = 0; w < WARPS; ++w) M = fmaxf(M, part.m[w][r]);
         float a = 0.f, ls = 0.f;
 #pragma unroll
         for (int w = 0; w < WARPS; ++w) {
-            const float f = s_m[w][r] == -INFINITY ? 0.f : __expf(s_m[w][r] - M);
-            a += f * s_acc[w][r][d];
-            ls += f * s_l[w][r];
+            const float f = part.m[w][r] == -INFINITY ? 0.f : __expf(part.m[w][r] - M);
+            a += f * part.acc[w][r][d];
+            ls += f * part.l[w][r];
         }
         c_acc[r][d] = a;
         if (d == 0) {

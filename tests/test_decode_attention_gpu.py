@@ -66,3 +66,39 @@ def test_gradients_keep_the_differentiable_path():
     g = torch.autograd.grad(attention(q, k, v, causal=True).float().square().sum(), (q, k, v))
     r = torch.autograd.grad(attention_reference(q, k, v, causal=True).float().square().sum(), (q, k, v))
     assert all(torch.equal(a, b) for a, b in zip(g, r))
+
+
+@pytest.mark.parametrize("Sk,D", [(2, 64), (40, 128), (1500, 128), (700, 64)])
+def test_values_that_are_not_finite_reach_the_rows_that_attend_to_them(Sk, D):
+    from lm_engine_b200.ops import attention, attention_reference
+
+    q, k, v = _inputs(2, Sk, 12, 2, D)
+    inf = float("inf")
+    v[0, Sk // 2, 0, 3] = inf
+    v[0, 0, 0, 9] = -inf
+    v[0, Sk - 1, 0, 17] = float("nan")
+    v[0, 0, 0, 33] = inf                                    # opposite infinities in one column: not a number
+    v[0, Sk - 1, 0, 33] = -inf
+    v[1, 1, 1, 0] = 3e38                                    # finite, with a finite average
+    out = attention(q, k, v, causal=True).float()
+    ref = attention_reference(q.double(), k.double(), v.double(), causal=True).double().float()
+    # weights of this many random keys stay far above the smallest fp32 number, so no product is 0 * inf
+    bad = ~torch.isfinite(ref)
+    assert bool(bad[0, 0, :6, [3, 9, 17, 33]].all()) and int(bad.sum()) == 24
+    torch.testing.assert_close(out[bad], ref[bad], rtol=0, atol=0, equal_nan=True)
+    for b in range(2):      # (the rounding of the result, 2^-9 per element)
+        o, r = (t[b].masked_fill(bad[b], 0.0).double() for t in (out, ref))
+        assert float((o - r).norm() / r.norm()) < 2.0 ** -8.5
+    o, r = (t[0].masked_fill(bad[0], 0.0) for t in (out, ref))
+    assert float((o - r).norm() / r.norm()) < 2.0 ** -8.5
+
+
+def test_values_behind_the_mask_are_not_read():
+    from lm_engine_b200.ops import attention
+
+    q, k, v = _inputs(2, 100, 8, 2, 128)
+    mask = torch.ones(2, 100, dtype=torch.bool, device="cuda")
+    mask[:, :40] = False
+    want = attention(q, k, v, causal=True, attention_mask=mask)
+    v[:, 7], v[:, 8], k[:, 9] = float("inf"), float("nan"), float("nan")
+    assert torch.equal(attention(q, k, v, causal=True, attention_mask=mask), want)
