@@ -541,8 +541,9 @@ __global__ void __launch_bounds__(256)
 ssd_boundary_fwd_kernel(const float* __restrict__ states, const float* __restrict__ decay,
                         const float* __restrict__ h_init, __nv_bfloat16* __restrict__ h0_bf16,
                         float* __restrict__ h0_f32, float* __restrict__ h_final, int NC, int N, int E) {
-    const int b = blockIdx.y / N, n = blockIdx.y - b * N;
-    const int e = (blockIdx.x * 256 + threadIdx.x) * 4;
+    const int slices = (E / 4 + 255) / 256, bn = blockIdx.x / slices, slice = blockIdx.x - bn * slices;
+    const int b = bn / N, n = bn - b * N;
+    const int e = (slice * 256 + threadIdx.x) * 4;
     if (e >= E) return;
     float4 h = make_float4(0.f, 0.f, 0.f, 0.f);
     if (h_init != nullptr) h = *reinterpret_cast<const float4*>(h_init + (static_cast<long long>(b) * N + n) * E + e);
@@ -568,9 +569,10 @@ __global__ void __launch_bounds__(256)
 ssd_boundary_bwd_kernel(const float* __restrict__ dh0, const float* __restrict__ dh_final,
                         const float* __restrict__ h0_f32, const float* __restrict__ decay, T* __restrict__ dstates,
                         float* __restrict__ ddecay_parts, int parts, float* __restrict__ dh_init, int NC, int N, int E) {
-    const int b = blockIdx.y / N, n = blockIdx.y - b * N;
-    const int e = (blockIdx.x * 256 + threadIdx.x) * 4;
-    const int part = (blockIdx.x * 256 + threadIdx.x) >> 5;
+    const int slices = (E / 4 + 255) / 256, bn = blockIdx.x / slices, slice = blockIdx.x - bn * slices;
+    const int b = bn / N, n = bn - b * N;
+    const int e = (slice * 256 + threadIdx.x) * 4;
+    const int part = (slice * 256 + threadIdx.x) >> 5;
     const bool in = e < E;
     float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
     if (in && dh_final != nullptr) g = *reinterpret_cast<const float4*>(dh_final + (static_cast<long long>(b) * N + n) * E + e);
@@ -604,8 +606,9 @@ ssd_boundary_bwd_kernel(const float* __restrict__ dh0, const float* __restrict__
 extern "C" int lme_ssd_boundary_fwd(const float* states, const float* decay, const float* h_init, void* h0_bf16,
                                     float* h0_f32, float* h_final, int B, int NC, int N, int E, void* stream) {
     if (B <= 0 || NC <= 0 || N <= 0 || E <= 0 || (E % 4)) return LME_ERR_SHAPE;
-    if (static_cast<long long>(B) * N > 65535) return LME_ERR_SHAPE;
-    lme::ssd_boundary_fwd_kernel<<<dim3((E / 4 + 255) / 256, B * N), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+    const long long blocks = static_cast<long long>(B) * N * ((E / 4 + 255) / 256);
+    if (blocks > 0x7fffffffll) return LME_ERR_SHAPE;
+    lme::ssd_boundary_fwd_kernel<<<static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
         states, decay, h_init, static_cast<__nv_bfloat16*>(h0_bf16), h0_f32, h_final, NC, N, E);
     return cudaGetLastError() == cudaSuccess ? LME_OK : LME_ERR_LAUNCH;
 }
@@ -614,9 +617,11 @@ extern "C" int lme_ssd_boundary_fwd(const float* states, const float* decay, con
 extern "C" int lme_ssd_boundary_bwd(const float* dh0, const float* dh_final, const float* h0_f32, const float* decay,
                                     void* dstates, int dstates_bf16, float* ddecay_parts, float* dh_init, int B, int NC,
                                     int N, int E, void* stream) {
-    if (B <= 0 || NC <= 0 || N <= 0 || E <= 0 || (E % 4) || static_cast<long long>(B) * N > 65535) return LME_ERR_SHAPE;
+    if (B <= 0 || NC <= 0 || N <= 0 || E <= 0 || (E % 4)) return LME_ERR_SHAPE;
+    const long long blocks = static_cast<long long>(B) * N * ((E / 4 + 255) / 256);
+    if (blocks > 0x7fffffffll) return LME_ERR_SHAPE;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const dim3 grid((E / 4 + 255) / 256, B * N);
+    const unsigned grid = static_cast<unsigned>(blocks);
     const int parts = (E + 127) / 128;
     if (dstates_bf16)
         lme::ssd_boundary_bwd_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(

@@ -137,7 +137,7 @@ class _BoundaryScan(torch.autograd.Function):
 def scan_glue_eligible(x: torch.Tensor, L: int, Sd: int) -> bool:
     b, S, N, P = x.shape
     return (x.is_cuda and x.dtype == torch.bfloat16 and L % 32 == 0 and L <= 1024 and P in (32, 64, 128)
-            and Sd % 8 == 0 and 0 < b * N <= 65535 and 0 < b * ((S + L - 1) // L) <= 65535 and FUSED_INTRA_CHUNK)
+            and Sd % 8 == 0 and b * N > 0 and 0 < b * ((S + L - 1) // L) <= 65535 and FUSED_INTRA_CHUNK)
 
 
 def _per_head(t: torch.Tensor, N: int) -> bool:

@@ -37,3 +37,27 @@ def test_a_step_width_that_does_not_fit_raises():
     with pytest.raises(RuntimeError):
         ssd_chunk_scan(x, torch.zeros(1, 32, 1, device="cuda"), -torch.ones(4, device="cuda"), B, B,
                        torch.ones(4, device="cuda"), 32)
+
+
+def test_more_sequences_times_heads_than_a_grid_dimension_holds():
+    from lm_engine_b200.ops import _lib
+    from lm_engine_b200.ops.ssd import ssd_chunk_scan
+
+    b, S, N, P, Sd = 2064, 40, 32, 32, 8
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x, B, C = (torch.randn(*s, generator=g, device="cuda").to(torch.bfloat16)
+               for s in ((b, S, N, P), (b, S, 1, Sd), (b, S, 1, Sd)))
+    dt, A, D = torch.rand(b, S, N, generator=g, device="cuda"), -torch.rand(N, generator=g, device="cuda"), torch.ones(N, device="cuda")
+
+    def run(s):
+        ins = [t[s].detach().requires_grad_(True) for t in (x, dt, B, C)]
+        before = _lib.launch_count
+        y, h = ssd_chunk_scan(ins[0], ins[1], A, ins[2], ins[3], D, 32)
+        grads = torch.autograd.grad((y.float().square().sum() + h.square().sum()), ins)
+        return _lib.launch_count - before, [y.detach(), h.detach(), *grads]
+
+    launches, whole = run(slice(0, b))
+    halves = [run(slice(0, b // 2)), run(slice(b // 2, b))]
+    assert launches == halves[0][0]                       # the same kernels
+    for i, t in enumerate(whole):
+        assert torch.equal(t, torch.cat([h[1][i] for h in halves]))
