@@ -134,10 +134,10 @@ class _BoundaryScan(torch.autograd.Function):
         return dstates, parts.sum(-1), dinit
 
 
-def scan_glue_eligible(x: torch.Tensor, L: int, Sd: int) -> bool:
+def scan_glue_eligible(x: torch.Tensor, L: int) -> bool:
     b, S, N, P = x.shape
     return (x.is_cuda and x.dtype == torch.bfloat16 and L % 32 == 0 and L <= 1024 and P in (32, 64, 128)
-            and Sd % 8 == 0 and b * N > 0 and 0 < b * ((S + L - 1) // L) <= 65535 and FUSED_INTRA_CHUNK)
+            and b * N > 0 and 0 < b * ((S + L - 1) // L) <= 65535 and FUSED_INTRA_CHUNK)
 
 
 def _per_head(t: torch.Tensor, N: int) -> bool:
@@ -167,7 +167,7 @@ def ssd_chunk_scan(x, dt, A, B, C, D, chunk_size: int, initial_state=None):
     dtype = x.dtype
     L = chunk_size
     pad = (L - S % L) % L
-    if scan_glue_eligible(x, L, Sd) and _per_head(A, N) and _per_head(D, N):
+    if scan_glue_eligible(x, L) and _per_head(A, N) and _per_head(D, N):
         return _chunk_scan_kernels(x, dt, A, B, C, D, L, initial_state)
     xf, dtf, Bf, Cf = x.float(), dt.float(), B.float(), C.float()
     if pad:
@@ -348,29 +348,39 @@ def _chunk_rows(t: torch.Tensor, bc: int, L: int) -> torch.Tensor:
 
 
 def _chunk_scan_kernels(x, dt, A, B, C, D, L: int, initial_state):
-    """Pads to whole chunks (padded steps have dt = 0: decay 1, no input) and runs :class:`_ChunkScan`.  The kernels
-    get bare addresses, so every operand takes its full shape here (a mismatch raises)."""
+    """Pads to whole chunks (padded steps have dt = 0: decay 1, no input) and the state to a multiple of 8 (zero columns
+    of B and C: the products read 16-byte rows), and runs :class:`_ChunkScan`.  The kernels get bare addresses, so every
+    operand takes its full shape here (a mismatch raises)."""
     b, S, N, P = x.shape
     G, Sd = B.shape[-2:]
     if N % G:
         raise ValueError(f"ssd: {N} heads do not split into {G} groups")
     bf = torch.bfloat16
     pad = (L - S % L) % L
-    B, C, dt = B.to(bf), C.to(bf), dt.float()
+
+    def shaped(t, *shape):      # a view of the same shape would be one more autograd node each way
+        return t if t.shape == shape else t.reshape(shape)
+
+    B, C, dt = shaped(B.to(bf), b, S, G, Sd), shaped(C.to(bf), b, S, G, Sd), shaped(dt.float(), b, S, N)
+    wide = -Sd % 8
+    if pad or wide:
+        B, C = (torch.nn.functional.pad(t, (0, wide, 0, 0, 0, pad)) for t in (B, C))
     if pad:
-        x, B, C = (torch.nn.functional.pad(t, (0, 0, 0, 0, 0, pad)) for t in (x, B, C))
-        dt = torch.nn.functional.pad(dt, (0, 0, 0, pad))
-    B, C, dt = B.reshape(b, S + pad, G, Sd), C.reshape(b, S + pad, G, Sd), dt.reshape(b, S + pad, N)
-    A, D = (t.float().reshape(-1).expand(N).contiguous() for t in (A, D))
+        x, dt = torch.nn.functional.pad(x, (0, 0, 0, 0, 0, pad)), torch.nn.functional.pad(dt, (0, 0, 0, pad))
+    A, D = (t.float() if t.shape == (N,) else t.float().reshape(-1).expand(N) for t in (A, D))
     if initial_state is not None:
-        initial_state = initial_state.expand(b, N, P, Sd)
+        if initial_state.shape != (b, N, P, Sd):
+            initial_state = initial_state.expand(b, N, P, Sd)
+        if wide:
+            initial_state = torch.nn.functional.pad(initial_state, (0, wide))
     # rows of x: heads contiguous inside a token, one pitch from token to token over the whole batch
     ok = (x.stride(3) == 1 and x.stride(2) == P and x.stride(1) % 8 == 0 and x.data_ptr() % 16 == 0
           and (b == 1 or x.stride(0) == x.size(1) * x.stride(1)))
     from ._lib import aligned
 
-    y, h = _ChunkScan.apply(x if ok else aligned(x), dt.contiguous(), A, B, C, D, L, initial_state)
-    return y[:, :S], h
+    y, h = _ChunkScan.apply(x if ok else aligned(x), dt.contiguous(), A.contiguous(), B, C,
+                            D.contiguous(), L, initial_state)
+    return y[:, :S], h[..., :Sd] if wide else h
 
 
 def ssd_context_parallel_initial_state(final_zero_init: torch.Tensor, total_decay: torch.Tensor, group) -> torch.Tensor:

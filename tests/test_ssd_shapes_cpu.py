@@ -56,3 +56,10 @@ def test_other_broadcasts_take_the_general_path(calls):
     ops = _operands(A=-torch.rand(L, N))                   # a decay per position of the chunk
     y, h = ssd.ssd_chunk_scan(**ops, chunk_size=L)
     assert not calls and y.shape == ops["x"].shape
+
+
+def test_states_of_any_width_reach_the_kernels(calls):
+    y, h = ssd.ssd_chunk_scan(**_operands(B=torch.zeros(b, S, G, 12), C=torch.zeros(b, S, G, 12),
+                                          initial_state=torch.zeros(b, N, P, 12)), chunk_size=L)
+    assert calls[0]["B"] == calls[0]["C"] == (b, 64, G, 16) and calls[0]["h"] == (b, N, P, 16)
+    assert h.shape == (b, N, P, 12)
