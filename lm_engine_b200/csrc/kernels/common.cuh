@@ -12,6 +12,8 @@
 #include <stdint.h>
 #include <type_traits>
 
+#include "opt_in.cuh"
+
 #ifndef LME_WAIT_LIMIT_NS
 #define LME_WAIT_LIMIT_NS 2000000000ull  // 2 s
 #endif

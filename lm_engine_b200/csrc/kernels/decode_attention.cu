@@ -267,12 +267,7 @@ __global__ void __launch_bounds__(WARPS * 32, 3) decode_attention_kernel(const _
 template <int D>
 static int launch_decode_attention(const Args& a, int B, int splits, cudaStream_t st) {
     auto kern = decode_attention_kernel<D>;
-    static int configured = 0;   // clusters of 16 need an opt-in
-    if (!configured) {
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
-            return LME_ERR_LAUNCH;
-        configured = 1;
-    }
+    if (!opt_in<decode_attention_kernel<D>>(cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) return LME_ERR_LAUNCH;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(splits, a.Hkv * a.head_blocks, B);
     cfg.blockDim = dim3(WARPS * 32);

@@ -691,12 +691,7 @@ static int check(const Rows& q, const Rows& k, const Rows& v, int B, int S, int 
 
 template <auto Kern, typename Args>
 static int launch(const Args& a, int threads, int smem, long long blocks, void* stream) {
-    static bool configured = false;
-    if (!configured) {
-        if (cudaFuncSetAttribute(Kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-            return LME_ERR_LAUNCH;
-        configured = true;
-    }
+    if (!opt_in<Kern>(cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) return LME_ERR_LAUNCH;
     Kern<<<static_cast<unsigned>(blocks), threads, smem, static_cast<cudaStream_t>(stream)>>>(a);
     return cudaGetLastError() == cudaSuccess ? LME_OK : LME_ERR_LAUNCH;
 }

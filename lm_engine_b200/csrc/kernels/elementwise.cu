@@ -776,16 +776,8 @@ static RowPlan row_plan(int H, int nt) {
     // warp rows: the weight-gradient sums of the warps (groups * H floats) fit two stages of two operands
     return p;
 }
-// raises a kernel's dynamic shared memory limit once (per size it grows to), not on every launch
-template <auto Kern>
-static int row_smem(int smem) {
-    static int have = 0;
-    if (smem <= have) return LME_OK;
-    if (cudaFuncSetAttribute(Kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-        return LME_ERR_LAUNCH;
-    have = smem;
-    return LME_OK;
-}
+// what the largest plan takes: two stages of three rows of 16384 columns, and the barriers
+static constexpr int ROW_SMEM_MAX = 2 * 3 * 16384 * 2 + 8 * 8;
 static inline int grid_for(long long work, int block, int cap) {
     long long g = (work + block - 1) / block;
     if (g < 1) g = 1;
@@ -840,7 +832,7 @@ extern "C" int lme_rmsnorm_fwd(const void* x, const void* residual, const void* 
     const int grid = grid_for((static_cast<long long>(T) + groups - 1) / groups, 1, LME_RMSNORM_BWD_MAX_PARTIAL_ROWS);
 #define LME_ROWS(VPT, WARP)                                                                             \
     do {                                                                                                \
-        if (int rc = row_smem<rmsnorm_fwd_kernel<VPT, WARP>>(plan.smem)) return rc;                     \
+        if (!opt_in<rmsnorm_fwd_kernel<VPT, WARP>>(cudaFuncAttributeMaxDynamicSharedMemorySize, ROW_SMEM_MAX)) return LME_ERR_LAUNCH; \
         rmsnorm_fwd_kernel<VPT, WARP><<<grid, plan.threads, plan.smem, st>>>(X, R, W, Y, HO, rstd, T, H, eps, plan.ring); \
     } while (0)
     LME_ROWS_DISPATCH();
@@ -873,7 +865,7 @@ extern "C" int lme_rmsnorm_bwd(const void* dy, const void* h, const void* w, con
     const RowPlan plan = row_plan(H, dres != nullptr ? 3 : 2);
 #define LME_ROWS(VPT, WARP)                                                                             \
     do {                                                                                                \
-        if (int rc = row_smem<rmsnorm_bwd_kernel<VPT, WARP>>(plan.smem)) return rc;                     \
+        if (!opt_in<rmsnorm_bwd_kernel<VPT, WARP>>(cudaFuncAttributeMaxDynamicSharedMemorySize, ROW_SMEM_MAX)) return LME_ERR_LAUNCH; \
         rmsnorm_bwd_kernel<VPT, WARP><<<G, plan.threads, plan.smem, st>>>(DY, HH, W, rstd, DR, DX, dw_partial, T, H, plan.ring); \
     } while (0)
     LME_ROWS_DISPATCH();

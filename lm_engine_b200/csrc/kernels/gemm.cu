@@ -886,12 +886,9 @@ template <int STAGES, bool A_MN, bool B_MN>
 static int launch_gemm_split_stages(const CUtensorMap& ta, const CUtensorMap& tb, GemmArgs& p, int splits,
                              cudaStream_t stream) {
     auto kern = gemm_split_kernel<STAGES, A_MN, B_MN>;
-    static bool configured = false;
-    if (!configured) {
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitLayout<STAGES>::TOTAL) != cudaSuccess)
-            return LME_ERR_LAUNCH;
-        configured = true;
-    }
+    if (!opt_in<gemm_split_kernel<STAGES, A_MN, B_MN>>(cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                       SplitLayout<STAGES>::TOTAL))
+        return LME_ERR_LAUNCH;
     p.tiles_m = (p.M + BM - 1) / BM;
     p.tiles_n = (p.N + SK_BN - 1) / SK_BN;
     p.group_m = 8;

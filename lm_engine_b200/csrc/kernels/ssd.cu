@@ -102,7 +102,7 @@ ssd_dcb_kernel(const __nv_bfloat16* __restrict__ dm, const float* __restrict__ c
 // at a time (the library's scan along an outer dimension takes 64 us for the same 1 MB; with 32 heads per CTA only 32
 // CTAs existed for 16 chunks x 64 heads and the reverse took 41 us).
 constexpr int DECAY_HEADS = 8;                       // one per warp
-constexpr int DECAY_LD = DECAY_HEADS + 1;
+constexpr int DECAY_LD = DECAY_HEADS + 1;           // at most 1024 rows of it: 36 KB
 
 __global__ void __launch_bounds__(256)
 ssd_decay_fwd_kernel(const float* __restrict__ dt, const float* __restrict__ A, float* __restrict__ ct,
@@ -437,7 +437,6 @@ extern "C" int lme_ssd_decay_fwd(const float* dt, const float* A, float* ct, flo
     if (BC <= 0) return LME_OK;
     if (L % 32 || L > 1024 || BC > 0x7fffffffll) return LME_ERR_SHAPE;
     const int smem = L * DECAY_LD * 4;
-    if (int rc = row_smem<ssd_decay_fwd_kernel>(smem)) return rc;
     ssd_decay_fwd_kernel<<<dim3(static_cast<unsigned>(BC), (N + DECAY_HEADS - 1) / DECAY_HEADS), 256, smem,
                            static_cast<cudaStream_t>(stream)>>>(dt, A, ct, dtt, tail, ecum, decay, N, L);
     return LME_LAUNCH_OK();
@@ -450,7 +449,6 @@ extern "C" int lme_ssd_decay_bwd(const float* dtt, const float* A, const float* 
     if (BC <= 0) return LME_OK;
     if (L % 32 || L > 1024 || BC > 0x7fffffffll) return LME_ERR_SHAPE;
     const int smem = L * DECAY_LD * 4;
-    if (int rc = row_smem<ssd_decay_bwd_kernel>(smem)) return rc;
     ssd_decay_bwd_kernel<<<dim3(static_cast<unsigned>(BC), (N + DECAY_HEADS - 1) / DECAY_HEADS), 256, smem,
                            static_cast<cudaStream_t>(stream)>>>(dtt, A, tail, ecum, decay, sy, decum, ddt0, sw,
                                                                 sh, ddecay_parts, parts, dDp, ddt, dA_part, dD_part, N,
