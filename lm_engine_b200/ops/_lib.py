@@ -165,6 +165,17 @@ def ptr(t: torch.Tensor | None) -> int | None:
     return None if t is None else t.data_ptr()
 
 
+def eager(*tensors: torch.Tensor) -> bool:
+    """Whether kernels may take these tensors by address: plain tensors of the current device, outside tracing,
+    functorch transforms, forward-mode AD and dispatch modes, all of which need operations that they can see."""
+    if (torch.compiler.is_compiling() or torch._C._is_tracing() or torch._C._len_torch_dispatch_stack()
+            or torch.autograd.forward_ad._current_level >= 0
+            or torch._C._functorch.peek_interpreter_stack() is not None):
+        return False
+    return all((type(t) is torch.Tensor or type(t) is torch.nn.Parameter) and t.is_cuda for t in tensors) and all(
+        t.get_device() == torch._C._cuda_getDevice() for t in tensors)
+
+
 def strides(t: torch.Tensor) -> tuple[int, ...]:
     """Element strides of ``t``, those of size-1 dimensions as in a dense tensor: PyTorch leaves them arbitrary and hands
     them through ``contiguous()`` and ``clone()``, so they say nothing about where elements are."""

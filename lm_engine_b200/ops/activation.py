@@ -96,40 +96,49 @@ def _row_pitch(t: torch.Tensor) -> int | None:
 
 
 class _SiLUMul(torch.autograd.Function):
+    """y dense, gate with one row pitch (:func:`silu_mul` sees to both)."""
+
     @staticmethod
     def forward(ctx, y, gate):
         I = y.size(-1)
-        y2 = _lib.aligned(y.reshape(-1, I))
-        out = torch.empty_like(y2)
-        _lib.check(_lib.cuda_lib().lme_silu_mul_fwd(y2.data_ptr(), gate.data_ptr(), _row_pitch(gate), out.data_ptr(),
-                                                    y2.size(0), I, _lib.stream_ptr()), "lme_silu_mul_fwd")
+        out = torch.empty(y.shape, dtype=y.dtype, device=y.device)
+        _lib.check(_lib.cuda_lib().lme_silu_mul_fwd(y.data_ptr(), gate.data_ptr(), _row_pitch(gate), out.data_ptr(),
+                                                    y.numel() // I, I, _lib.stream_ptr()), "lme_silu_mul_fwd")
         _lib.count_launch()
-        ctx.save_for_backward(y2, gate)
-        ctx.shape = y.shape
-        return out.view(y.shape)
+        ctx.save_for_backward(y, gate)
+        return out
 
     @staticmethod
     def backward(ctx, dout):
-        y2, gate = ctx.saved_tensors
+        y, gate = ctx.saved_tensors
+        if torch.is_grad_enabled():         # a graph of the gradients is asked for
+            y, gate = y.view_as(y), gate.view_as(gate)
+            wrt = [t for t, needed in zip((y, gate), ctx.needs_input_grad) if needed]
+            grads = iter(torch.autograd.grad(_silu_mul_statement(y, gate), wrt, dout, create_graph=True))
+            return tuple(next(grads) if needed else None for needed in ctx.needs_input_grad)
+        y, dout = _lib.aligned(y), _lib.aligned(dout)
         if _row_pitch(gate) is None:        # a saved-tensor hook may return other strides
             gate = _lib.aligned(gate)
-        T, I = y2.shape
-        d2 = _lib.aligned(dout.reshape(T, I))
-        dy, dg = torch.empty_like(y2), torch.empty_like(y2)
-        _lib.check(_lib.cuda_lib().lme_silu_mul_bwd(d2.data_ptr(), y2.data_ptr(), gate.data_ptr(), _row_pitch(gate),
-                                                    dy.data_ptr(), dg.data_ptr(), T, I, _lib.stream_ptr()),
-                   "lme_silu_mul_bwd")
+        I = y.size(-1)
+        dy, dg = (torch.empty(y.shape, dtype=y.dtype, device=y.device) for _ in range(2))
+        _lib.check(_lib.cuda_lib().lme_silu_mul_bwd(dout.data_ptr(), y.data_ptr(), gate.data_ptr(), _row_pitch(gate),
+                                                    dy.data_ptr(), dg.data_ptr(), y.numel() // I, I,
+                                                    _lib.stream_ptr()), "lme_silu_mul_bwd")
         _lib.count_launch()
-        return dy.view(ctx.shape), dg.view(gate.shape)
+        return dy, dg
 
 
 def _silu_mul_kernel_usable(y: torch.Tensor, gate: torch.Tensor) -> bool:
-    return (y.is_cuda and gate.is_cuda and y.dtype == gate.dtype == torch.bfloat16 and y.shape == gate.shape
-            and y.dim() >= 2 and y.size(-1) % 8 == 0 and y.numel() > 0)
+    return (y.dtype == gate.dtype == torch.bfloat16 and y.shape == gate.shape and y.dim() >= 2
+            and y.size(-1) % 8 == 0 and y.numel() > 0 and _lib.eager(y, gate))
+
+
+def _silu_mul_statement(y, gate):
+    return y * torch.nn.functional.silu(gate.float()).to(gate.dtype)
 
 
 def silu_mul(y: torch.Tensor, gate: torch.Tensor) -> torch.Tensor:
     """``y * silu(gate)``, the activation rounded to its input type; ``gate`` may be a slice of wider rows."""
     if _silu_mul_kernel_usable(y, gate):
-        return _SiLUMul.apply(y, gate if _row_pitch(gate) is not None else _lib.aligned(gate))
-    return y * torch.nn.functional.silu(gate.float()).to(gate.dtype)
+        return _SiLUMul.apply(_lib.aligned(y), gate if _row_pitch(gate) is not None else _lib.aligned(gate))
+    return _silu_mul_statement(y, gate)

@@ -48,18 +48,17 @@ def decode_supported(q, k, v, *, causal, sliding_window, attention_mask, cu_seql
     """One new token per sequence over a longer cache, outside autograd (generation): the case that would otherwise
     run as the PyTorch statement, which expands K and V to fp32 copies per query head.  One key, or a plain
     non-causal call, keeps the library path that it has."""
-    if not (type(q) is type(k) is type(v) is torch.Tensor and q.is_cuda and q.dim() == 4 and q.size(1) == 1
+    if not (q.is_cuda and q.dim() == 4 and q.size(1) == 1
             and q.dtype == k.dtype == v.dtype == torch.bfloat16 and q.size(-1) in (64, 128)
             and k.dim() == 4 and k.shape == v.shape and q.size(-1) == k.size(-1) and q.size(0) == k.size(0)
             and k.size(2) > 0 and q.size(2) % k.size(2) == 0 and dropout_p == 0 and cu_seqlens is None):
         return False
     if torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad):
         return False
-    if attention_mask is not None and not (type(attention_mask) is torch.Tensor and attention_mask.is_cuda
-                                           and attention_mask.shape == (k.size(0), k.size(1))):
+    if attention_mask is not None and attention_mask.shape != (k.size(0), k.size(1)):
         return False
-    if torch.autograd.forward_ad._current_level >= 0 or torch._C._functorch.peek_interpreter_stack() is not None:
-        return False        # transforms see the statement
+    if not _lib.eager(q, k, v, *(() if attention_mask is None else (attention_mask,))):
+        return False
     plain = sliding_window is None and attention_mask is None
     return (k.size(1) > 1 and not (plain and not causal) and (sliding_window is None or sliding_window > 0)
             and q.size(0) <= 65535 and k.size(2) * ((q.size(2) // k.size(2) + 7) // 8) <= 65535)
@@ -71,11 +70,12 @@ def decode_attention(q, k, v, *, softmax_scale: float, sliding_window: int | Non
     nothing are zero; values of hidden keys are not read into the sum."""
     def rows(t):
         *pitches, inner = _lib.strides(t)
-        ok = inner == 1 and t.data_ptr() % 16 == 0 and not any(p % 8 for p in pitches)
-        return t if ok else _lib.aligned(t)
+        if inner == 1 and t.data_ptr() % 16 == 0 and not any(p % 8 for p in pitches):
+            return t, *pitches
+        t = _lib.aligned(t)
+        return t, *_lib.strides(t)[:3]
 
-    q, k, v = rows(q), rows(k), rows(v)
-    (q_b, _, q_h, _), (k_b, k_s, k_h, _), (v_b, v_s, v_h, _) = (_lib.strides(t) for t in (q, k, v))
+    (q, q_b, _, q_h), (k, k_b, k_s, k_h), (v, v_b, v_s, v_h) = rows(q), rows(k), rows(v)
     B, _, Hq, D = q.shape
     Sk, Hkv = k.size(1), k.size(2)
     out = torch.empty((B, 1, Hq, D), dtype=q.dtype, device=q.device)

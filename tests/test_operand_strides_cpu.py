@@ -72,6 +72,21 @@ def test_gate_rows(lib, monkeypatch, name):
             assert 0 <= (ptr - base) // 2 and (ptr - base) // 2 + (T - 1) * pitch + I <= n
 
 
+@pytest.mark.parametrize("wrt", [(0, 1), (0,), (1,)])
+def test_gradients_of_the_gate_s_gradients(lib, monkeypatch, wrt):
+    from lm_engine_b200.ops import activation
+
+    monkeypatch.setattr(activation, "_silu_mul_kernel_usable", lambda y, gate: True)
+    ins = [torch.randn(3, 16).to(BF).requires_grad_(i in wrt) for i in range(2)]
+    dout, dd, results = torch.randn(3, 16).to(BF).requires_grad_(True), torch.randn(3, 16).to(BF), []
+    for f in (activation.silu_mul, activation._silu_mul_statement):
+        first = torch.autograd.grad(f(*ins), [ins[i] for i in wrt], dout, create_graph=True)
+        second = torch.autograd.grad(first, [dout, *(ins[i] for i in wrt)], [dd] * len(wrt), allow_unused=True)
+        results.append([*first, *(t for t in second if t is not None)])
+    assert len(results[0]) == len(results[1]) >= 2 * len(wrt)
+    assert all(torch.equal(a, b) for a, b in zip(*results))
+
+
 ROWS = {
     # x [B, S, C], element strides (batch, time) of an in-place read at four taps; None: a dense copy
     "one row, odd width": (lambda: _wide(1, 1, 1001, 8, 16), (16, 16)),
