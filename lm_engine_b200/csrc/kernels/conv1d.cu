@@ -284,11 +284,11 @@ __device__ __forceinline__ void conv4_filter(const Conv4& p, int c, float (&w)[4
 
 __global__ void __launch_bounds__(128, 8) causal_conv4_fwd_kernel(const Conv4 p, __nv_bfloat16* __restrict__ y) {
     constexpr int V = 4;
-    // blockIdx.x: channel groups of one time run after the other (runs of 16 steps do not fit grid.y beyond a million steps)
-    const int groups = (p.C / V + 127) / 128, run = blockIdx.x / groups;
-    const int c = ((blockIdx.x - run * groups) * 128 + threadIdx.x) * V;
+    // time runs in grid.x: runs of 16 steps do not fit another dimension beyond a million steps
+    const int run = blockIdx.x;
+    const int c = (blockIdx.y * 128 + threadIdx.x) * V;
     if (c >= p.C) return;
-    const long long b = blockIdx.y;
+    const long long b = blockIdx.z;
     const int t0 = run * CONV4_STEPS, t1 = min(t0 + CONV4_STEPS, p.S);
     float w[4][V], bv[V], x0[V], x1[V], x2[V];
     conv4_filter(p, c, w, bv);
@@ -464,9 +464,7 @@ extern "C" int lme_causal_conv1d_fwd(const void* x, long long x_b, long long x_t
     if (K == 4) {
         if (reinterpret_cast<uintptr_t>(w) & 7) return LME_ERR_ALIGN;
         const Conv4 p{X, W, BI, IN, x_b, x_t, S, C, silu};
-        const long long blocks = static_cast<long long>((C / 4 + 127) / 128) * ((S + CONV4_STEPS - 1) / CONV4_STEPS);
-        if (blocks > 0x7fffffffll) return LME_ERR_SHAPE;
-        causal_conv4_fwd_kernel<<<dim3(static_cast<unsigned>(blocks), B), 128, 0, st>>>(p, Y);
+        causal_conv4_fwd_kernel<<<dim3((S + CONV4_STEPS - 1) / CONV4_STEPS, (C / 4 + 127) / 128, B), 128, 0, st>>>(p, Y);
     } else if (K < 4) causal_conv1d_fwd_kernel<4><<<grid, 128, 0, st>>>(X, W, BI, IN, Y, B, S, C, K, silu);
     else causal_conv1d_fwd_kernel<CONV_MAX_K><<<grid, 128, 0, st>>>(X, W, BI, IN, Y, B, S, C, K, silu);
     return cudaGetLastError() == cudaSuccess ? LME_OK : LME_ERR_LAUNCH;
