@@ -179,11 +179,15 @@ def eager(*tensors: torch.Tensor) -> bool:
 def strides(t: torch.Tensor) -> tuple[int, ...]:
     """Element strides of ``t``, those of size-1 dimensions as in a dense tensor: PyTorch leaves them arbitrary and hands
     them through ``contiguous()`` and ``clone()``, so they say nothing about where elements are."""
-    out, dense = [], 1
-    for size, stride in zip(reversed(t.shape), reversed(t.stride())):
-        out.append(dense if size == 1 else stride)
-        dense *= size
-    return tuple(reversed(out))
+    shape, out = t.shape, t.stride()
+    if 1 not in shape:
+        return out
+    out, dense = list(out), 1
+    for d in range(len(out) - 1, -1, -1):
+        if shape[d] == 1:
+            out[d] = dense
+        dense *= shape[d]
+    return tuple(out)
 
 
 def aligned(t: torch.Tensor) -> torch.Tensor:

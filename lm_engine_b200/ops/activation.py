@@ -95,14 +95,20 @@ def _row_pitch(t: torch.Tensor) -> int | None:
     return pitch if pitch % 8 == 0 and pitch >= t.size(-1) else None
 
 
+def _rows(t: torch.Tensor) -> tuple[torch.Tensor, int]:
+    """``t`` with its row pitch, copied where it has none."""
+    pitch = _row_pitch(t)
+    return (_lib.aligned(t), t.size(-1)) if pitch is None else (t, pitch)
+
+
 class _SiLUMul(torch.autograd.Function):
     """y dense, gate with one row pitch (:func:`silu_mul` sees to both)."""
 
     @staticmethod
-    def forward(ctx, y, gate):
+    def forward(ctx, y, gate, pitch):
         I = y.size(-1)
         out = torch.empty(y.shape, dtype=y.dtype, device=y.device)
-        _lib.check(_lib.cuda_lib().lme_silu_mul_fwd(y.data_ptr(), gate.data_ptr(), _row_pitch(gate), out.data_ptr(),
+        _lib.check(_lib.cuda_lib().lme_silu_mul_fwd(y.data_ptr(), gate.data_ptr(), pitch, out.data_ptr(),
                                                     y.numel() // I, I, _lib.stream_ptr()), "lme_silu_mul_fwd")
         _lib.count_launch()
         ctx.save_for_backward(y, gate)
@@ -116,16 +122,15 @@ class _SiLUMul(torch.autograd.Function):
             wrt = [t for t, needed in zip((y, gate), ctx.needs_input_grad) if needed]
             grads = iter(torch.autograd.grad(_silu_mul_statement(y, gate), wrt, dout, create_graph=True))
             return tuple(next(grads) if needed else None for needed in ctx.needs_input_grad)
+        gate, pitch = _rows(gate)           # (a saved-tensor hook may return other strides)
         y, dout = _lib.aligned(y), _lib.aligned(dout)
-        if _row_pitch(gate) is None:        # a saved-tensor hook may return other strides
-            gate = _lib.aligned(gate)
         I = y.size(-1)
         dy, dg = (torch.empty(y.shape, dtype=y.dtype, device=y.device) for _ in range(2))
-        _lib.check(_lib.cuda_lib().lme_silu_mul_bwd(dout.data_ptr(), y.data_ptr(), gate.data_ptr(), _row_pitch(gate),
+        _lib.check(_lib.cuda_lib().lme_silu_mul_bwd(dout.data_ptr(), y.data_ptr(), gate.data_ptr(), pitch,
                                                     dy.data_ptr(), dg.data_ptr(), y.numel() // I, I,
                                                     _lib.stream_ptr()), "lme_silu_mul_bwd")
         _lib.count_launch()
-        return dy, dg
+        return dy, dg, None
 
 
 def _silu_mul_kernel_usable(y: torch.Tensor, gate: torch.Tensor) -> bool:
@@ -140,5 +145,5 @@ def _silu_mul_statement(y, gate):
 def silu_mul(y: torch.Tensor, gate: torch.Tensor) -> torch.Tensor:
     """``y * silu(gate)``, the activation rounded to its input type; ``gate`` may be a slice of wider rows."""
     if _silu_mul_kernel_usable(y, gate):
-        return _SiLUMul.apply(_lib.aligned(y), gate if _row_pitch(gate) is not None else _lib.aligned(gate))
+        return _SiLUMul.apply(_lib.aligned(y), *_rows(gate))
     return _silu_mul_statement(y, gate)

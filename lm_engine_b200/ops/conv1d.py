@@ -7,6 +7,8 @@ from __future__ import annotations
 import torch
 import torch.nn.functional as F
 
+from . import _lib
+
 
 def causal_conv1d_reference(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None,
                             initial_state: torch.Tensor | None, activation: str | None) -> torch.Tensor:
@@ -28,8 +30,6 @@ def causal_conv1d_reference(x: torch.Tensor, weight: torch.Tensor, bias: torch.T
 def _rows(x: torch.Tensor, K: int) -> tuple[torch.Tensor, int, int]:
     """x with its batch and time strides as the kernels take them: the four-tap kernels read a slice of wider rows in
     place (16-byte rows), everything else is a dense copy."""
-    from . import _lib
-
     x_b, x_t, x_c = _lib.strides(x)
     if K != 4 or x_c != 1 or x_t % 8 or x_b % 8 or x.data_ptr() % 16:
         x = _lib.aligned(x)
@@ -42,8 +42,6 @@ class _CausalConv1d(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, weight, bias, initial_state, silu: bool):
-        from . import _lib
-
         B, S, C = x.shape
         K = weight.size(1)
         x, x_b, x_t = _rows(x, K)
@@ -60,8 +58,6 @@ class _CausalConv1d(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy):
-        from . import _lib
-
         x, w, bias, init = ctx.saved_tensors
         B, S, C = x.shape
         K = w.size(1)

@@ -142,7 +142,7 @@ def scan_glue_eligible(x: torch.Tensor, L: int) -> bool:
 
 def _per_head(t: torch.Tensor, N: int) -> bool:
     """One value per head, or one for all; other shapes that broadcast take the general path."""
-    return t.numel() in (1, N) and t.shape[-1:].numel() == t.numel()
+    return t.shape == (N,) or (t.numel() in (1, N) and t.shape[-1:].numel() == t.numel())
 
 
 def _intra_chunk_fused(Cc, Bc, ct, xdt):
@@ -357,11 +357,9 @@ def _chunk_scan_kernels(x, dt, A, B, C, D, L: int, initial_state):
         raise ValueError(f"ssd: {N} heads do not split into {G} groups")
     bf = torch.bfloat16
     pad = (L - S % L) % L
-
-    def shaped(t, *shape):      # a view of the same shape would be one more autograd node each way
-        return t if t.shape == shape else t.reshape(shape)
-
-    B, C, dt = shaped(B.to(bf), b, S, G, Sd), shaped(C.to(bf), b, S, G, Sd), shaped(dt.float(), b, S, N)
+    B, C, dt = B.to(bf), C.to(bf), dt.float()
+    if not (B.shape == C.shape == (b, S, G, Sd) and dt.shape == (b, S, N)):
+        B, C, dt = B.reshape(b, S, G, Sd), C.reshape(b, S, G, Sd), dt.reshape(b, S, N)
     wide = -Sd % 8
     if pad or wide:
         B, C = (torch.nn.functional.pad(t, (0, wide, 0, 0, 0, pad)) for t in (B, C))
