@@ -282,11 +282,13 @@ __device__ __forceinline__ void conv4_filter(const Conv4& p, int c, float (&w)[4
     }
 }
 
-__global__ void __launch_bounds__(128, 8) causal_conv4_fwd_kernel(const Conv4 p, __nv_bfloat16* __restrict__ y) {
+// Channel groups in grid.x and time runs in grid.y: blocks that run together read whole rows (22.3 us at 4096 steps x 4352
+// channels, 23.3 with the two exchanged).  More runs than grid.y holds, a million steps, exchange them all the same.
+__global__ void __launch_bounds__(128, 8)
+causal_conv4_fwd_kernel(const Conv4 p, __nv_bfloat16* __restrict__ y, const bool exchanged) {
     constexpr int V = 4;
-    // time runs in grid.x: runs of 16 steps do not fit another dimension beyond a million steps
-    const int run = blockIdx.x;
-    const int c = (blockIdx.y * 128 + threadIdx.x) * V;
+    const int run = exchanged ? blockIdx.x : blockIdx.y;
+    const int c = ((exchanged ? blockIdx.y : blockIdx.x) * 128 + threadIdx.x) * V;
     if (c >= p.C) return;
     const long long b = blockIdx.z;
     const int t0 = run * CONV4_STEPS, t1 = min(t0 + CONV4_STEPS, p.S);
@@ -464,7 +466,9 @@ extern "C" int lme_causal_conv1d_fwd(const void* x, long long x_b, long long x_t
     if (K == 4) {
         if (reinterpret_cast<uintptr_t>(w) & 7) return LME_ERR_ALIGN;
         const Conv4 p{X, W, BI, IN, x_b, x_t, S, C, silu};
-        causal_conv4_fwd_kernel<<<dim3((S + CONV4_STEPS - 1) / CONV4_STEPS, (C / 4 + 127) / 128, B), 128, 0, st>>>(p, Y);
+        const int runs = (S + CONV4_STEPS - 1) / CONV4_STEPS, groups = (C / 4 + 127) / 128;
+        const bool exchanged = runs > 65535;
+        causal_conv4_fwd_kernel<<<exchanged ? dim3(runs, groups, B) : dim3(groups, runs, B), 128, 0, st>>>(p, Y, exchanged);
     } else if (K < 4) causal_conv1d_fwd_kernel<4><<<grid, 128, 0, st>>>(X, W, BI, IN, Y, B, S, C, K, silu);
     else causal_conv1d_fwd_kernel<CONV_MAX_K><<<grid, 128, 0, st>>>(X, W, BI, IN, Y, B, S, C, K, silu);
     return cudaGetLastError() == cudaSuccess ? LME_OK : LME_ERR_LAUNCH;
