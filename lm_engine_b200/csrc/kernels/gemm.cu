@@ -973,7 +973,7 @@ extern "C" int lme_gemm_bf16(const void* A, int a_mn_major, long long lda, const
     p.scale_a = p.scale_b = nullptr;
     if (max_ctas <= 0) max_ctas = num_sms();
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-if (splits > 0) {
+    if (splits > 0) {
         if (a_mn_major && b_mn_major) return launch_gemm_split<true, true>(ta, tb, p, splits, st);
         if (a_mn_major) return launch_gemm_split<true, false>(ta, tb, p, splits, st);
         if (b_mn_major) return launch_gemm_split<false, true>(ta, tb, p, splits, st);

@@ -85,10 +85,6 @@ def sigmoid(x: torch.Tensor) -> torch.Tensor:
     return torch.sigmoid(x.float()).to(x.dtype)
 
 
-def silu(x: torch.Tensor) -> torch.Tensor:
-    return torch.nn.functional.silu(x.float()).to(x.dtype)
-
-
 def tanh(x: torch.Tensor) -> torch.Tensor:
     return torch.tanh(x.float()).to(x.dtype)
 

@@ -83,7 +83,6 @@ def cuda_lib() -> ctypes.CDLL:
             "lme_moe_route_layout": [P, I, I, P, P, P, P, P, I, P, P],
             "lme_delta_prep_fwd": [P, P, P, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, F, P],
             "lme_delta_prep_bwd": [P, P, P, P, P, P, P, P, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, F, P],
-            "lme_decode_attention": [P, L, L, P, L, L, L, P, L, L, L, P, L, P, I, I, I, I, I, I, F, P],
             "lme_delta_chain_fwd": [P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, P],
             "lme_delta_chain_bwd": [P, P, P, P, P, P, P, P, P, P, I, I, I, I, P],
             "lme_causal_conv1d_fwd": [P, L, L, P, P, P, P, I, I, I, I, I, P],

@@ -94,7 +94,8 @@ class _IntraChunk(torch.autograd.Function):
 class _BoundaryScan(torch.autograd.Function):
     """``h_{c+1} = decay[c] h_c + S_c`` over the chunks of every (batch, head) in one kernel each way.  Returns the
     state at every chunk start in bf16 (``[b, nc, N, P, Sd]``, the operand of the carried-state product) and the
-    final state in fp32."""
+    final state in fp32.  By itself: gradients of the states in fp32; :class:`_ChunkScan` runs the same kernels with
+    gradients in the type that its products read."""
 
     @staticmethod
     def forward(ctx, states, decay, h_init):
