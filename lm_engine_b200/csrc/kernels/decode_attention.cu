@@ -15,7 +15,7 @@
 // tcgen05 has nothing to add: one row per head is used, and the bound is HBM.
 // Measured (24 sequences x 3001 keys, 8 K / V heads of 128, 295 MB): 76 us = 3.9 TB/s (84 us without the loads one block
 // ahead); the PyTorch statement that served this case before expands K and V to one fp32 copy per query head and took
-// 2640 us.  What is left is latency: 12 warps per SM at 168 registers, a third of the issue slots used.
+// 2640 us.  What is left is latency: 12 warps per SM at 168 registers, a quarter of the issue slots used.
 // Included by lme_cuda.cu after m2rnn.cu (mma helper).
 
 namespace lme {
@@ -310,8 +310,9 @@ extern "C" int lme_decode_attention(const void* q, long long q_b, long long q_h,
     a.head_blocks = (G + 7) / 8;
     a.scale = scale;
     if (B > 65535 || static_cast<long long>(Hkv) * a.head_blocks > 65535) return LME_ERR_SHAPE;
-    // The keys are split until there is a CTA for every slot of the chip (three fit an SM), but no slice is shorter than
-    // the 64 keys that the four warps take in one step: a slice costs a prologue and a merge of about 4 us.
+    // The keys are split until there is a CTA for every slot of the chip (three fit an SM), and no further once a slice is
+    // down to the 64 keys that the four warps take in one step: a slice costs a prologue and a merge of about 4 us.  Slices
+    // therefore keep more than 32 keys (48 with the rounding to blocks of 16); the last ones get what is left, or nothing.
     const long long rows = static_cast<long long>(B) * Hkv * a.head_blocks;
     int splits = 1;
     while (splits < lme::da::MAX_SPLITS && rows * splits < 3 * 148 && (Sk - a.first) > splits * 64) splits *= 2;

@@ -928,6 +928,9 @@ static int launch_gemm_split(const CUtensorMap& ta, const CUtensorMap& tb, GemmA
 // Four as long as all CTAs are resident at two per SM with room to spare, two while they are and K is long enough to
 // pay for the sum (or one per SM), one while every tile has an SM; from there on the wider tiles of the persistent
 // kernel.  Clusters of eight only won where a whole GPC was free for each and lost elsewhere.
+// The number of shares follows from M, and each share is accumulated by itself: a row's product is the same in every
+// repetition, but its last fp32 bits depend on how many other rows there are (a prompt and a generation step of the same
+// token differ by the rounding) and on whether the caller limits the CTAs.
 static int gemm_splits(int M, int N, int K) {
     const long long tiles = static_cast<long long>((M + BM - 1) / BM) * ((N + SK_BN - 1) / SK_BN);
     const int blocks = (K + BK - 1) / BK, sms = num_sms();
