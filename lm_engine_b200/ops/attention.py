@@ -113,9 +113,10 @@ def attention(q, k, v, *, causal=True, softmax_scale=None, sliding_window=None, 
         return attention_cuda.flash_attention(q, k, v, causal=causal, softmax_scale=scale,
                                               sliding_window=sliding_window, cu_seqlens=cu_seqlens,
                                               max_seqlen=max_seqlen)
-    if attention_cuda.decode_supported(q, k, v, causal=causal, sliding_window=sliding_window,
-                                       attention_mask=attention_mask, cu_seqlens=cu_seqlens, dropout_p=dropout_p):
-        return attention_cuda.decode_attention(q, k, v, softmax_scale=scale, sliding_window=sliding_window,
+    if not isinstance(scale, torch.Tensor) and attention_cuda.decode_supported(
+            q, k, v, causal=causal, sliding_window=sliding_window, attention_mask=attention_mask, cu_seqlens=cu_seqlens,
+            dropout_p=dropout_p):
+        return attention_cuda.decode_attention(q, k, v, softmax_scale=float(scale), sliding_window=sliding_window,
                                                attention_mask=attention_mask)
     if q.is_cuda:
         from ..logging_utils.logger import warn_once

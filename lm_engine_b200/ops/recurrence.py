@@ -454,8 +454,9 @@ def gated_delta_rule(q, k, v, g, beta, scale=None, h0=None, use_qk_l2norm: bool 
     if q.size(1) < 8:
         return gated_delta_rule_scan(q, k, v, g, beta, scale, h0, use_qk_l2norm)
     if q.is_cuda and q.size(-1) in (128, 256) and v.size(-1) % 64 == 0:
-        # the chain over 64-step blocks is one kernel each way, and so is the block-local part on bf16 inputs
-        if gated_delta_blocks_usable(q, k, v, g, beta):
+        # the chain over 64-step blocks is one kernel each way, and so is the block-local part on bf16 inputs (a scale
+        # that is a tensor may want its gradient)
+        if not isinstance(scale, torch.Tensor) and gated_delta_blocks_usable(q, k, v, g, beta):
             return gated_delta_rule_blocks(q, k, v, g, beta, scale, h0, use_qk_l2norm)
         return gated_delta_rule_chunked(q, k, v, g, beta, scale, h0, use_qk_l2norm, chunk=64)
     # the loop over blocks is the sequential (launch-bound) part and the block-local work is cheap: long sequences
