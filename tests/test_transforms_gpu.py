@@ -57,3 +57,55 @@ def test_transforms_of_the_gate():
     f64 = torch.autograd.grad(ins[0] * torch.nn.functional.silu(ins[1]), ins, dy64, create_graph=True)
     for a, b in zip(second, torch.autograd.grad(f64, ins, (dg64, dg64))):
         assert float((a.double() - b).norm() / b.norm()) < 2.0 ** -6
+
+
+def test_saved_tensors_that_come_back_with_other_strides():
+    from lm_engine_b200.ops import silu_mul
+    from lm_engine_b200.ops.conv1d import causal_conv1d
+    from lm_engine_b200.ops.recurrence import gated_delta_rule
+    from lm_engine_b200.ops.ssd import ssd_chunk_scan
+
+    g = torch.Generator(device="cuda").manual_seed(0)
+
+    def r(*s):
+        return torch.randn(*s, generator=g, device="cuda").to(BF).requires_grad_(True)
+
+    wide, w, y = r(2, 70, 1024), r(512, 4), r(2, 70, 512)
+    f = (-0.1 * torch.rand(2, 70, 2, generator=g, device="cuda")).requires_grad_(True)
+
+    def heads(a, b, n):
+        return wide[..., a:b].unflatten(-1, (n, -1))
+
+    one = torch.ones(4, device="cuda")
+    cases = {
+        "gate": (lambda: silu_mul(y, wide[..., 512:]), (y, wide)),
+        "convolution": (lambda: causal_conv1d(wide[..., 512:], w, None, None, "silu"), (wide, w)),
+        "delta rule": (lambda: gated_delta_rule(heads(0, 256, 2), heads(256, 512, 2), heads(512, 640, 2), f, -f)[0],
+                       (wide, f)),
+        "scan": (lambda: ssd_chunk_scan(heads(0, 128, 4), -f.repeat(1, 1, 2), -one, heads(128, 144, 1),
+                                        heads(144, 160, 1), one, 32)[0], (wide, f)),
+    }
+    moved = []
+
+    def pack(t):            # slices come back as rows of another pitch
+        if t.dim() < 3 or t.is_leaf or t.is_contiguous():
+            return t, False
+        moved.append(t.shape)
+        return torch.nn.functional.pad(t, (0, 3)), True
+
+    for name, (run, wrt) in cases.items():
+        out = run()
+        dout = torch.randn(out.shape, generator=g, device="cuda").to(out.dtype)
+        want = torch.autograd.grad(out, wrt, dout)
+        with torch.autograd.graph.save_on_cpu():
+            dense = run()
+        results = [torch.autograd.grad(dense, wrt, dout)]
+        if name != "scan":      # (the scan takes whole chunks as dense copies here)
+            moved.clear()
+            with torch.autograd.graph.saved_tensors_hooks(pack, lambda p: p[0][..., :-3] if p[1] else p[0]):
+                padded = run()
+            assert moved, name
+            results.append(torch.autograd.grad(padded, wrt, dout))
+        for got in results:     # equal but for the convolution's weight gradient, which is added in any order
+            for a, b in zip(got, want):
+                assert float((a.double() - b.double()).norm() / b.double().norm()) < 2.0 ** -8, name
